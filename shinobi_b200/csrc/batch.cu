@@ -15,7 +15,7 @@
 #include <chrono>
 
 #include "internal.h"
-#include "trace_coop.cuh"
+#include "trace_flat.cuh"
 
 struct shn_batch {
   shn_ctx* ctx = nullptr;
@@ -64,20 +64,16 @@ namespace {
 
 constexpr int kBatchTraceBlock = 128;
 
+// All scenes' cells and triangles are one array each; triangles are read by
+// id through indices[].
 struct BatchAcc {
+  static constexpr bool kIndirect = true;
   const BatchScene* sc;
-  const uint2* cells;
-  SHN_D const Geom& geom(uint32_t s) const { return sc[s].g; }
-  SHN_D const uint2* cells_of(uint32_t s) const { return cells + sc[s].cell_offset; }
-};
-
-struct BatchAccW {
-  static constexpr bool kIndirect = true;  // no reference-ordered copy: triangles through indices[]
-  BatchAcc a;
+  const uint2* all;
   Refs r;
-  SHN_D const Geom& geom(uint32_t s) const { return a.geom(s); }
-  SHN_D const uint2* cells(uint32_t s) const { return a.cells_of(s); }
-  SHN_D const uint2* leaves(uint32_t) const { return nullptr; }
+  SHN_D const Geom& geom(uint32_t s) const { return sc[s].g; }
+  SHN_D const uint2* cells(uint32_t) const { return all; }
+  SHN_D uint32_t cell0(uint32_t s) const { return (uint32_t)sc[s].cell_offset; }
   SHN_D Refs refs(uint32_t) const { return r; }
 };
 
@@ -86,15 +82,15 @@ struct RaysV {
 };
 
 template <bool ANY>
-__global__ void __launch_bounds__(kBatchTraceBlock, 8) k_batch_trace(GridView G, BatchAcc A, RaysV R,
-                                                                 const uint32_t* __restrict__ ray_off,
+__global__ void __launch_bounds__(kBatchTraceBlock, kFlatBlocks) k_batch_trace(GridView G, const BatchScene* scenes, const uint2* cells,
+                                                                 RaysV R, const uint32_t* __restrict__ ray_off,
                                                                  uint32_t ns, uint32_t n, uint32_t* counter,
                                                                  uint32_t* otri, float* ot, float* ou,
                                                                  float* ov, uint8_t* occ) {
-  // incoherent rays rarely share a cell range: no grouping (measured slower here)
-  warp_trace_acc<0, ANY, false>(
-      BatchAccW{A, refs_of(G)}, n, counter,
-      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t& scene, uint32_t&) {
+  __shared__ FlatWarp sm[kBatchTraceBlock / 32];
+  flat_trace<ANY>(
+      sm, BatchAcc{scenes, cells, refs_of(G)}, n, ou || ov, counter,
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t& scene) {
         uint32_t lo = 0, hi = ns;
         while (hi - lo > 1) {
           const uint32_t mid = (lo + hi) >> 1;
@@ -105,11 +101,11 @@ __global__ void __launch_bounds__(kBatchTraceBlock, 8) k_batch_trace(GridView G,
         d = mk(R.dx[i], R.dy[i], R.dz[i]);
         tmax = R.tmax ? R.tmax[i] : FLT_MAX;
       },
-      [&](uint32_t i, const Hit& h, uint32_t, uint32_t, uint32_t scene) {
+      [&](uint32_t i, const Hit& h, uint32_t scene) {
         if (ANY) {
           occ[i] = h.tri != kMiss ? 1 : 0;
         } else {
-          otri[i] = h.tri == kMiss ? kMiss : h.tri - A.sc[scene].tri_offset;
+          otri[i] = h.tri == kMiss ? kMiss : h.tri - scenes[scene].tri_offset;
           ot[i] = h.t;
           if (ou) ou[i] = h.u;
           if (ov) ov[i] = h.v;
@@ -256,13 +252,12 @@ void enqueue_trace(shn_batch* b, const shn_rays* rays, uint32_t n, shn_hits* hit
                    cudaStream_t st) {
   cudaMemsetAsync(b->d_counter, 0, 4, st);
   const GridView G = batch_view(b);
-  const BatchAcc A{b->d_scenes, b->cells};
   const RaysV R{rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmax};
   if (occ) {
-    k_batch_trace<true><<<b->blocks_any, kBatchTraceBlock, 0, st>>>(G, A, R, b->d_ray_off, b->ns, n, b->d_counter,
+    k_batch_trace<true><<<b->blocks_any, kBatchTraceBlock, 0, st>>>(G, b->d_scenes, b->cells, R, b->d_ray_off, b->ns, n, b->d_counter,
                                                              nullptr, nullptr, nullptr, nullptr, occ);
   } else {
-    k_batch_trace<false><<<b->blocks_closest, kBatchTraceBlock, 0, st>>>(G, A, R, b->d_ray_off, b->ns, n, b->d_counter,
+    k_batch_trace<false><<<b->blocks_closest, kBatchTraceBlock, 0, st>>>(G, b->d_scenes, b->cells, R, b->d_ray_off, b->ns, n, b->d_counter,
                                                               hits->tri, hits->t, hits->u, hits->v, nullptr);
   }
 }

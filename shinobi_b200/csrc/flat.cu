@@ -1,0 +1,122 @@
+// Trace kernels of uniform grids on the flat engine: rays from arrays, camera
+// rays, and the any-hit rays made from a frame's primary hits.
+#include "internal.h"
+#include "rays.cuh"
+#include "trace_flat.cuh"
+
+namespace shn {
+
+namespace {
+
+struct RaysView {
+  const float *ox, *oy, *oz, *dx, *dy, *dz, *tmax;
+};
+
+template <bool ANY>
+__global__ void __launch_bounds__(kCoopBlock, kFlatBlocks) k_flat_rays(const __grid_constant__ GridView G, RaysView R, uint32_t n, uint32_t* counter,
+                                                           uint32_t* otri, float* ot, float* ou, float* ov,
+                                                           uint8_t* occ) {
+  __shared__ FlatWarp sm[kCoopBlock / 32];
+  flat_trace<ANY>(
+      sm, FlatGrid{&G}, n, ou || ov, counter,
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) {
+        o = mk(__ldg(R.ox + i), __ldg(R.oy + i), __ldg(R.oz + i));
+        d = mk(__ldg(R.dx + i), __ldg(R.dy + i), __ldg(R.dz + i));
+        tmax = R.tmax ? __ldg(R.tmax + i) : FLT_MAX;
+      },
+      [&](uint32_t i, const Hit& h, uint32_t) {
+        if (ANY) {
+          occ[i] = h.tri != kMiss ? 1 : 0;
+        } else {
+          otri[i] = h.tri;
+          ot[i] = h.t;
+          if (ou) ou[i] = h.u;
+          if (ov) ov[i] = h.v;
+        }
+      });
+}
+
+__global__ void __launch_bounds__(kCoopBlock, kFlatBlocks) k_flat_camera(const __grid_constant__ GridView G, CamView cam, uint32_t image_id, uint32_t n,
+                                                             uint32_t* counter, uint32_t* otri, float* ot, float* ou,
+                                                             float* ov) {
+  __shared__ FlatWarp sm[kCoopBlock / 32];
+  flat_trace<false>(
+      sm, FlatGrid{&G}, n, ou || ov, counter,
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) {
+        o = cam.eye;
+        d = primary_dir(cam, tile_pixel(cam, i), image_id);
+        tmax = FLT_MAX;
+      },
+      [&](uint32_t r, const Hit& h, uint32_t) {
+        const uint32_t i = tile_pixel(cam, r);
+        otri[i] = h.tri;
+        ot[i] = h.t;
+        if (ou) ou[i] = h.u;
+        if (ov) ov[i] = h.v;
+      });
+}
+
+template <class Rays>
+__global__ void __launch_bounds__(kCoopBlock, kFlatBlocks) k_flat_from_hits(const __grid_constant__ GridView G,
+                                                                         const __grid_constant__ Rays R,
+                                                                         const uint32_t* d_m, uint32_t spp,
+                                                                         uint32_t* counter) {
+  __shared__ FlatWarp sm[kCoopBlock / 32];
+  flat_trace<true>(
+      sm, FlatGrid{&G}, (*d_m) * spp, false, counter,
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) { R.ray(i, o, d, tmax); },
+      [&](uint32_t i, const Hit& h, uint32_t) { R.done(i, h); });
+}
+
+// Persistent blocks, no more than one warp per ray needs.
+template <class K>
+int flat_blocks(K kernel, int num_sms, uint64_t n) {
+  static const int per_sm = [&] {
+    int v = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, kCoopBlock, 0);
+    return std::max(1, v);
+  }();
+  const uint64_t need = (n + kCoopBlock / 32 - 1) / (kCoopBlock / 32);
+  return (int)std::min<uint64_t>((uint64_t)per_sm * num_sms, need);
+}
+
+RaysView view(const shn_rays& r) { return RaysView{r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.tmax}; }
+
+}  // namespace
+
+void launch_flat_closest(const GridView& G, const shn_rays& rays, uint32_t n, uint32_t* counter, const shn_hits& hits,
+                         int num_sms, cudaStream_t st) {
+  k_flat_rays<false><<<flat_blocks(k_flat_rays<false>, num_sms, n), kCoopBlock, 0, st>>>(
+      G, view(rays), n, counter, hits.tri, hits.t, hits.u, hits.v, nullptr);
+}
+
+void launch_flat_any(const GridView& G, const shn_rays& rays, uint32_t n, uint32_t* counter, uint8_t* occ, int num_sms,
+                     cudaStream_t st) {
+  k_flat_rays<true><<<flat_blocks(k_flat_rays<true>, num_sms, n), kCoopBlock, 0, st>>>(
+      G, view(rays), n, counter, nullptr, nullptr, nullptr, nullptr, occ);
+}
+
+void launch_flat_camera(const GridView& G, const CamView& cam, uint32_t image_id, uint32_t n, uint32_t* counter,
+                        const shn_hits& hits, int num_sms, cudaStream_t st) {
+  k_flat_camera<<<flat_blocks(k_flat_camera, num_sms, n), kCoopBlock, 0, st>>>(G, cam, image_id, n, counter, hits.tri,
+                                                                             hits.t, hits.u, hits.v);
+}
+
+template <class Rays>
+static void from_hits(const GridView& G, const Rays& R, const uint32_t* d_m, uint32_t spp, uint32_t* counter,
+                      uint64_t most, int num_sms, cudaStream_t st) {
+  k_flat_from_hits<Rays><<<flat_blocks(k_flat_from_hits<Rays>, num_sms, most), kCoopBlock, 0, st>>>(G, R, d_m, spp,
+                                                                                                   counter);
+}
+
+void launch_flat_from_hits(const GridView& G, const AoRays& R, const uint32_t* d_m, uint32_t spp, uint32_t* counter,
+                           uint64_t most, int num_sms, cudaStream_t st) {
+  from_hits(G, R, d_m, spp, counter, most, num_sms, st);
+}
+
+void launch_flat_from_hits(const GridView& G, const DiRays& R, const uint32_t* d_m, uint32_t spp, uint32_t* counter,
+                           uint64_t most, int num_sms, cudaStream_t st) {
+  from_hits(G, R, d_m, spp, counter, most, num_sms, st);
+}
+
+}  // namespace shn

@@ -186,7 +186,24 @@ void launch_ranges(const uint64_t* keys, uint32_t n, uint2* ranges, uint32_t* in
 
 // trace.cu
 struct CamView;
+struct GridView;
 CamView make_camera(const shn_camera* c);
+GridView view_of(const shn_grid* g);
+
+// flat.cu: uniform grids; counter is a zeroed device word
+void launch_flat_closest(const GridView& G, const shn_rays& rays, uint32_t n, uint32_t* counter, const shn_hits& hits,
+                         int num_sms, cudaStream_t st);
+void launch_flat_any(const GridView& G, const shn_rays& rays, uint32_t n, uint32_t* counter, uint8_t* occ, int num_sms,
+                     cudaStream_t st);
+struct AoRays;
+struct DiRays;
+// d_m: number of hit pixels, on the device; most: an upper bound of the rays
+void launch_flat_from_hits(const GridView& G, const AoRays& R, const uint32_t* d_m, uint32_t spp, uint32_t* counter,
+                           uint64_t most, int num_sms, cudaStream_t st);
+void launch_flat_from_hits(const GridView& G, const DiRays& R, const uint32_t* d_m, uint32_t spp, uint32_t* counter,
+                           uint64_t most, int num_sms, cudaStream_t st);
+void launch_flat_camera(const GridView& G, const CamView& cam, uint32_t image_id, uint32_t n, uint32_t* counter,
+                        const shn_hits& hits, int num_sms, cudaStream_t st);
 
 // scan.cu (context-level primitives)
 // withhold_first: failure-detection self test -- the launch leaves out tile 0

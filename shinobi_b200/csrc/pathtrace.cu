@@ -1,11 +1,17 @@
-// Wavefront path tracer with stream compaction after every bounce.
+// Wavefront path tracer.
 //
 // The reference runs its path tracer as a persistent megakernel in which
 // finished paths leave their lanes idle until the whole warp is done
 // (src/Integrator/SimplePathTracer.hpp:65-241, src/Shinobi.h:152-230).  Here
-// every bounce is one persistent trace+shade kernel over the live paths,
-// followed by a decoupled look-back compaction that packs the survivors
-// (64-byte records) for the next bounce, so warps only ever see live paths.
+// every bounce is three kernels over the live paths: the extension rays, the
+// shading (which packs the survivors for the next bounce and lists the shadow
+// rays), and the shadow rays.
+//
+// What bounds it: the incoherent rays' walk.  One kernel that traced a path's
+// extension and shadow ray lane by lane ran at 3.5-4.7 of 32 lanes after the
+// first bounce; the trace kernels of uniform grids run the flat engine at
+// 17-26 lanes (4.2M-triangle heightfield, 1920 x 1080 x 16 paths, depth 4: 100 ->
+// 51 ms, of which the shading is 2.6 ms).
 //
 // Semantics (restated by the oracle path for path):
 //  * path g = sample * npix + (the pixel's number in 8x4-tile order); camera ray through the pixel with a
@@ -21,7 +27,8 @@
 //    per-pixel mean over samples summed in sample order (deterministic).
 // Random numbers: Philox4x32-10, counter (pixel, sample, depth, tag), key (seed, 0).
 #include "internal.h"
-#include "trace.cuh"
+#include "trace_coop.cuh"
+#include "trace_flat.cuh"
 
 namespace shn {
 
@@ -40,16 +47,27 @@ struct PtView {
   uint32_t snt;
 };
 
-// Path record: r0 = org.xyz, beta.x; r1 = dir.xyz, beta.y; r2 = L.xyz, beta.z;
-// r3 = (pixel, sample, depth, 0) bits.
+// Path record: org, beta.x | dir, beta.y | beta.z, pixel, sample.  Its
+// radiance accumulates in the path's slot.  Once shaded, a record whose path
+// has a shadow ray holds that: origin, c.x | segment, c.y | c.z, pixel,
+// sample, where c is added to the slot if the segment is free.
 struct PathRec {
-  float4 r0, r1, r2, r3;
+  float4 r0, r1, r2;
 };
 
-__global__ void k_pt_camera(PtView P, uint64_t g0, uint32_t count, PathRec* __restrict__ out,
-                            uint32_t* d_n) {
+struct PtHit {
+  float t;
+  uint32_t tri;
+};
+
+// Per bounce: live paths, shadow rays, work counters of the two trace kernels.
+struct PtCount {
+  uint32_t live, shadow, work0, work1;
+};
+
+__global__ void k_pt_camera(PtView P, uint64_t g0, uint32_t count, PathRec* __restrict__ out, PtCount* cnt) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k == 0) *d_n = count;
+  if (k == 0) cnt->live = count;
   if (k >= count) return;
   const uint64_t g = g0 + k;
   // path g = sample s, camera ray number g - s * npix, numbered by 8x4 pixel
@@ -67,121 +85,177 @@ __global__ void k_pt_camera(PtView P, uint64_t g0, uint32_t count, PathRec* __re
   PathRec r;
   r.r0 = make_float4(c.eye.x, c.eye.y, c.eye.z, 1.f);
   r.r1 = make_float4(d.x, d.y, d.z, 1.f);
-  r.r2 = make_float4(0.f, 0.f, 0.f, 1.f);
-  r.r3 = make_float4(__uint_as_float(p), __uint_as_float(s), __uint_as_float(0u), 0.f);
+  r.r2 = make_float4(1.f, __uint_as_float(p), __uint_as_float(s), 0.f);
   out[k] = r;
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(kPtBlock, 10) k_pt_bounce(GridView G, PtView P, PathRec* __restrict__ paths,
-                                                        const uint32_t* d_n, uint32_t depth,
-                                                        uint32_t* counter, uint32_t* __restrict__ alive,
-                                                        float4* __restrict__ slots, uint64_t g0,
-                                                        uint32_t* d_shadow) {
-  const uint32_t n = *d_n;
-  const int lane = threadIdx.x & 31;
-  uint32_t shadow_rays = 0;
-  while (true) {
-    uint32_t b = 0;
-    if (lane == 0) b = atomicAdd(counter, 32u);
-    const uint32_t base = __shfl_sync(0xFFFFFFFFu, b, 0);
-    if (base >= n) break;
-    const uint32_t i = base + lane;
-    if (i >= n) continue;
-    PathRec r = paths[i];
-    const V3 org = mk(r.r0.x, r.r0.y, r.r0.z);
-    const V3 dir = mk(r.r1.x, r.r1.y, r.r1.z);
-    V3 beta = mk(r.r0.w, r.r1.w, r.r2.w);
-    V3 L = mk(r.r2.x, r.r2.y, r.r2.z);
-    const uint32_t p = __float_as_uint(r.r3.x), s = __float_as_uint(r.r3.y);
-    if (p >= P.npix || s >= P.spp) {  // record left unwritten by a look-back that gave up
-      alive[i] = 0u;
-      continue;
-    }
-    Hit h{FLT_MAX, kMiss, 0.f, 0.f};
-    trace_ray<KIND, false>(G, org, dir, h);
-    bool live = false;
-    if (h.tri == kMiss) {
-      L = add(L, mul(beta, P.bg));
-    } else {
-      const float4* rec = P.stri + 3 * (size_t)h.tri;
-      const V3 v0 = f4v(__ldg(rec));
-      const V3 v1 = f4v(__ldg(rec + 1));
-      const V3 v2 = f4v(__ldg(rec + 2));
-      const V3 e1 = sub(v1, v0);
-      V3 nn = normalize(cross(e1, sub(v2, v0)));
-      if (dot(nn, dir) > 0.f) nn = mk(-nn.x, -nn.y, -nn.z);
-      const V3 hp = add(org, muls(dir, h.t));
-      const V3 o = add(hp, muls(nn, P.offset));
-      // next-event estimation
-      const uint4 wl = philox4x32(make_uint4(p, s, depth, kTagLight), P.seed, 0u);
-      const float lu = u01(wl.x), lv = u01(wl.y), urr = u01(wl.z);
-      const V3 lp = add(add(P.lpos, muls(P.le1, lu)), muls(P.le2, lv));
-      const V3 wv = sub(lp, o);
-      const float d2 = dot(wv, wv);
-      const V3 l = muls(wv, 1.0f / sqrtf(d2));
-      const float cs = dot(nn, l);
-      const float cl = -dot(P.lnrm, l);
-      if (cs > 0.f && cl > 0.f) {
-        Hit sh{0.9999f, kMiss, 0.f, 0.f};
-        trace_ray<KIND, true>(G, o, wv, sh);
-        ++shadow_rays;
-        if (sh.tri == kMiss) {
+// Extension rays of the live paths.
+struct PtExtend {
+  const PathRec* paths;
+  PtHit* hits;
+  SHN_D void ray(uint32_t i, V3& o, V3& d, float& tmax) const {
+    const float4 a = paths[i].r0, b = paths[i].r1;
+    o = f4v(a);
+    d = f4v(b);
+    tmax = FLT_MAX;
+  }
+  SHN_D void done(uint32_t i, const Hit& h) const { hits[i] = PtHit{h.t, h.tri}; }
+};
+
+// Shadow rays: rays[k] is the record that holds the k-th.
+struct PtShadow {
+  const PathRec* paths;
+  const uint32_t* rays;
+  float4* slots;
+  uint32_t npix;
+  SHN_D void ray(uint32_t k, V3& o, V3& d, float& tmax) const {
+    const PathRec& r = paths[rays[k]];
+    o = f4v(r.r0);
+    d = f4v(r.r1);
+    tmax = 0.9999f;
+  }
+  SHN_D void done(uint32_t k, const Hit& h) const {
+    if (h.tri != kMiss) return;
+    const PathRec& r = paths[rays[k]];
+    const float4 c = r.r2;
+    float4* s = slots + ((uint64_t)__float_as_uint(c.z) * npix + __float_as_uint(c.y));
+    const V3 L = add(f4v(*s), mk(r.r0.w, r.r1.w, c.x));
+    *s = make_float4(L.x, L.y, L.z, 0.f);
+  }
+};
+
+template <bool ANY, class Rays>
+__global__ void __launch_bounds__(kPtBlock, kFlatBlocks) k_pt_flat(const __grid_constant__ GridView G, Rays R, const uint32_t* n,
+                                                         uint32_t* counter) {
+  __shared__ FlatWarp sm[kPtBlock / 32];
+  flat_trace<ANY>(
+      sm, FlatGrid{&G}, *n, false, counter,
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) { R.ray(i, o, d, tmax); },
+      [&](uint32_t i, const Hit& h, uint32_t) { R.done(i, h); });
+}
+
+// Two-level grids.  Camera rays are taken as packets.
+template <bool ANY, bool PACKET, class Rays>
+__global__ void __launch_bounds__(kPtBlock, ANY ? 6 : 8) k_pt_two_level(GridView G, Rays R, const uint32_t* n,
+                                                              uint32_t* counter) {
+  warp_trace<1, ANY, PACKET>(
+      G, *n, counter, [&](uint32_t i, V3& o, V3& d, float& tmax) { R.ray(i, o, d, tmax); },
+      [&](uint32_t i, const Hit& h, uint32_t, uint32_t) { R.done(i, h); });
+}
+
+// Shades the live paths: light sample, roulette, next direction.  Survivors are
+// packed into `out` and shadow rays listed by blocks of paths, one addition to
+// each count per block; the order of the blocks does not show in the image.
+constexpr int kShadeBlock = 256;
+
+__global__ void __launch_bounds__(kShadeBlock) k_pt_shade(PtView P, PathRec* __restrict__ paths,
+                                                          const PtHit* __restrict__ hits, PathRec* __restrict__ out,
+                                                          uint32_t* __restrict__ shadow, uint32_t depth,
+                                                          PtCount* cnt, float4* __restrict__ slots) {
+  __shared__ uint32_t s_live[kShadeBlock / 32], s_shadow[kShadeBlock / 32];
+  const uint32_t n = cnt->live;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  for (uint32_t i0 = blockIdx.x * kShadeBlock; i0 < n; i0 += gridDim.x * kShadeBlock) {
+    const uint32_t i = i0 + threadIdx.x;
+    bool live = false, casts = false;
+    PathRec r, sh;
+    if (i < n) {
+      r = paths[i];
+      const PtHit h = hits[i];
+      const V3 org = f4v(r.r0), dir = f4v(r.r1);
+      V3 beta = mk(r.r0.w, r.r1.w, r.r2.x);
+      const uint32_t p = __float_as_uint(r.r2.y), s = __float_as_uint(r.r2.z);
+      float4* slot = slots + ((uint64_t)s * P.npix + p);
+      if (h.tri == kMiss) {
+        const V3 L = add(depth ? f4v(*slot) : mk(0.f, 0.f, 0.f), mul(beta, P.bg));
+        *slot = make_float4(L.x, L.y, L.z, 0.f);
+      } else {
+        if (depth == 0) *slot = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4* rec = P.stri + 3 * (size_t)h.tri;
+        const V3 v0 = f4v(__ldg(rec));
+        const V3 v1 = f4v(__ldg(rec + 1));
+        const V3 v2 = f4v(__ldg(rec + 2));
+        const V3 e1 = sub(v1, v0);
+        V3 nn = normalize(cross(e1, sub(v2, v0)));
+        if (dot(nn, dir) > 0.f) nn = mk(-nn.x, -nn.y, -nn.z);
+        const V3 hp = add(org, muls(dir, h.t));
+        const V3 o = add(hp, muls(nn, P.offset));
+        // next-event estimation
+        const uint4 wl = philox4x32(make_uint4(p, s, depth, kTagLight), P.seed, 0u);
+        const float lu = u01(wl.x), lv = u01(wl.y), urr = u01(wl.z);
+        const V3 lp = add(add(P.lpos, muls(P.le1, lu)), muls(P.le2, lv));
+        const V3 wv = sub(lp, o);
+        const float d2 = dot(wv, wv);
+        const V3 l = muls(wv, 1.0f / sqrtf(d2));
+        const float cs = dot(nn, l);
+        const float cl = -dot(P.lnrm, l);
+        if (cs > 0.f && cl > 0.f) {
           const float f = ((((P.albedo * 0.31830988618379067f) * cs) * cl) * P.larea) / d2;
-          L = add(L, muls(mul(beta, P.lrad), f));
+          const V3 c = muls(mul(beta, P.lrad), f);
+          casts = true;
+          sh.r0 = make_float4(o.x, o.y, o.z, c.x);
+          sh.r1 = make_float4(wv.x, wv.y, wv.z, c.y);
+          sh.r2 = make_float4(c.z, r.r2.y, r.r2.z, 0.f);
+        }
+        // continuation
+        live = depth + 1 < P.max_depth;
+        if (live && depth >= P.rr_depth) {
+          if (urr < P.albedo) beta = muls(beta, 1.0f / P.albedo);
+          else live = false;
+        }
+        if (live) {
+          const uint4 wd = philox4x32(make_uint4(p, s, depth, kTagDir), P.seed, 0u);
+          const float u1 = u01(wd.x), u2 = u01(wd.y);
+          float sn, cn;
+          sincos_2pi(u1, sn, cn);
+          const float rr = sqrtf(1.f - u2);
+          const float lx = sn * rr, ly = cn * rr, lz = sqrtf(u2);
+          const V3 tx = normalize(e1);
+          const V3 ty = cross(nn, tx);
+          const V3 nd = mk(tx.x * lx + ty.x * ly + nn.x * lz, tx.y * lx + ty.y * ly + nn.y * lz,
+                           tx.z * lx + ty.z * ly + nn.z * lz);
+          beta = muls(beta, P.albedo);
+          r.r0 = make_float4(o.x, o.y, o.z, beta.x);
+          r.r1 = make_float4(nd.x, nd.y, nd.z, beta.y);
+          r.r2.x = beta.z;
         }
       }
-      // continuation
-      live = depth + 1 < P.max_depth;
-      if (live && depth >= P.rr_depth) {
-        if (urr < P.albedo) beta = muls(beta, 1.0f / P.albedo);
-        else live = false;
-      }
-      if (live) {
-        const uint4 wd = philox4x32(make_uint4(p, s, depth, kTagDir), P.seed, 0u);
-        const float u1 = u01(wd.x), u2 = u01(wd.y);
-        float sn, cn;
-        sincos_2pi(u1, sn, cn);
-        const float rr = sqrtf(1.f - u2);
-        const float lx = sn * rr, ly = cn * rr, lz = sqrtf(u2);
-        const V3 tx = normalize(e1);
-        const V3 ty = cross(nn, tx);
-        const V3 nd = mk(tx.x * lx + ty.x * ly + nn.x * lz, tx.y * lx + ty.y * ly + nn.y * lz,
-                         tx.z * lx + ty.z * ly + nn.z * lz);
-        beta = muls(beta, P.albedo);
-        r.r0 = make_float4(o.x, o.y, o.z, beta.x);
-        r.r1 = make_float4(nd.x, nd.y, nd.z, beta.y);
-        r.r2 = make_float4(L.x, L.y, L.z, beta.z);
-        r.r3.z = __uint_as_float(depth + 1);
-        paths[i] = r;
-      }
     }
-    alive[i] = live ? 1u : 0u;
-    if (!live) slots[(uint64_t)s * P.npix + p - g0] = make_float4(L.x, L.y, L.z, 0.f);
-  }
-  if (d_shadow) {  // every lane leaves the loop at the same iteration
-    const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, shadow_rays);
-    if (lane == 0 && c) atomicAdd(d_shadow, c);
+    const uint32_t lm = __ballot_sync(0xFFFFFFFFu, live), cm = __ballot_sync(0xFFFFFFFFu, casts);
+    if (lane == 0) {
+      s_live[warp] = __popc(lm);
+      s_shadow[warp] = __popc(cm);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      uint32_t* w = threadIdx.x == 0 ? s_live : s_shadow;
+      uint32_t sum = 0;
+      for (int k = 0; k < kShadeBlock / 32; ++k) {
+        const uint32_t v = w[k];
+        w[k] = sum;
+        sum += v;
+      }
+      const uint32_t at = sum ? atomicAdd(threadIdx.x == 0 ? &cnt[1].live : &cnt->shadow, sum) : 0u;
+      for (int k = 0; k < kShadeBlock / 32; ++k) w[k] += at;
+    }
+    __syncthreads();
+    if (live) out[s_live[warp] + __popc(lm & lt)] = r;
+    if (casts) {
+      paths[i] = sh;
+      shadow[s_shadow[warp] + __popc(cm & lt)] = i;
+    }
+    __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(256) k_pt_compact(const PathRec* __restrict__ in,
-                                                    const uint32_t* __restrict__ alive,
-                                                    const uint32_t* d_n, PathRec* __restrict__ out,
-                                                    uint32_t* d_next, LookbackState st) {
-  __shared__ TileScanSmem<256, 8> sm;
-  const uint32_t n = *d_n;
-  // one tile per block; blocks beyond the live count only publish nothing
-  if ((uint64_t)blockIdx.x * 2048 >= n) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *d_next = 0;
-    return;
+__global__ void k_pt_stats(const PtCount* cnt, uint32_t depth, uint32_t* stats) {
+  uint32_t shadow = 0;
+  for (uint32_t d = 0; d < depth; ++d) {
+    stats[d] += cnt[d].live;
+    shadow += cnt[d].shadow;
   }
-  tile_scan<256, 8>(
-      st, n, sm, [&](uint32_t i) { return alive[i]; },
-      [&](uint32_t i, uint32_t ex) {
-        if (alive[i]) out[ex] = in[i];
-      },
-      d_next);
+  stats[depth] += shadow;
 }
 
 __global__ void k_pt_resolve(const float4* __restrict__ slots, uint32_t npix, uint32_t spp,
@@ -200,8 +274,29 @@ __global__ void k_pt_resolve(const float4* __restrict__ slots, uint32_t npix, ui
   img[3 * (size_t)p + 2] = b / (float)spp;
 }
 
-__global__ void k_copy_u32(const uint32_t* src, uint32_t* dst) { *dst = *src; }
-__global__ void k_add_u32(const uint32_t* src, uint32_t* dst) { *dst += *src; }
+template <class K>
+int pt_blocks(K kernel, int num_sms) {
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPtBlock, 0);
+  return std::max(1, per_sm) * num_sms;
+}
+
+// Extension (Rays = PtExtend) or shadow rays of one bounce.
+template <bool ANY, class Rays>
+void launch_rays(const GridView& G, const Rays& R, bool camera, const uint32_t* n, uint32_t* counter, uint32_t most,
+                 int num_sms, cudaStream_t st) {
+  const int need = (int)std::min<uint32_t>((most + kPtBlock / 32 - 1) / (kPtBlock / 32), 1u << 20);
+  if (G.kind == SHN_GRID_UNIFORM) {
+    static const int blocks = pt_blocks(k_pt_flat<ANY, Rays>, num_sms);
+    k_pt_flat<ANY, Rays><<<std::min(blocks, need), kPtBlock, 0, st>>>(G, R, n, counter);
+  } else if (!ANY && camera) {
+    static const int blocks = pt_blocks(k_pt_two_level<ANY, true, Rays>, num_sms);
+    k_pt_two_level<ANY, true, Rays><<<blocks, kPtBlock, 0, st>>>(G, R, n, counter);
+  } else {
+    static const int blocks = pt_blocks(k_pt_two_level<ANY, false, Rays>, num_sms);
+    k_pt_two_level<ANY, false, Rays><<<blocks, kPtBlock, 0, st>>>(G, R, n, counter);
+  }
+}
 
 }  // namespace
 
@@ -261,85 +356,50 @@ shn_status shn_pt_render(const shn_grid* g, const shn_scene* s, const shn_camera
   P.lnrm = normalize(ln);
   P.stri = s->tri;
   P.snt = s->nt;
-  const GridView G = [&] {
-    GridView v;
-    v.g = g->geom;
-    v.kind = g->kind;
-    v.cells = g->cells;
-    v.leaves = g->leaves;
-    v.rv0 = g->rtri;
-    v.rv1 = g->rtri + g->num_refs;
-    v.rv2 = g->rtri + 2 * g->num_refs;
-    v.src = g->src_tri;
-    v.cbox = g->num_blocks ? (const float4*)g->cbox.ptr : nullptr;
-    v.sbox = g->num_blocks ? (const float4*)g->sbox.ptr : nullptr;
-    v.ridx = nullptr;
-    return v;
-  }();
+  const GridView G = view_of(g);
 
-  // Waves of at most kWave paths bound the state memory (2 x 64 B per path + slots).
+  // Waves of at most kWave paths bound the state memory (108 bytes per path,
+  // and 16 per sample of the image).
   const uint64_t kWave = 1ull << 23;
   const uint32_t wave = (uint32_t)std::min<uint64_t>(total, kWave);
-  const size_t tiles = (wave + 2047) / 2048;
-  void *pa = nullptr, *pb = nullptr, *alive = nullptr, *slots = nullptr, *cnt = nullptr, *status = nullptr;
-  const size_t bRec = (size_t)wave * sizeof(PathRec), bAl = (size_t)wave * 4, bSl = (size_t)total * 16,
-               bCnt = 64 * 4, bSt = (tiles + 2) * 8;
-  cudaError_t e = dev_alloc(ctx, &pa, bRec, st);
-  if (e == cudaSuccess) e = dev_alloc(ctx, &pb, bRec, st);
-  if (e == cudaSuccess) e = dev_alloc(ctx, &alive, bAl, st);
-  if (e == cudaSuccess) e = dev_alloc(ctx, &slots, bSl, st);
-  if (e == cudaSuccess) e = dev_alloc(ctx, &cnt, bCnt, st);
-  if (e == cudaSuccess) e = dev_alloc(ctx, &status, bSt, st);
-  auto release = [&] {
-    dev_free(ctx, pa, bRec, st);
-    dev_free(ctx, pb, bRec, st);
-    dev_free(ctx, alive, bAl, st);
-    dev_free(ctx, slots, bSl, st);
-    dev_free(ctx, cnt, bCnt, st);
-    dev_free(ctx, status, bSt, st);
+  size_t bytes = 0;
+  const auto part = [&](size_t b) {
+    const size_t at = bytes;
+    bytes += (b + 255) & ~(size_t)255;
+    return at;
   };
-  if (e != cudaSuccess) {
-    release();
+  const size_t bCnt = ((size_t)prm->max_depth + 1) * sizeof(PtCount);
+  const size_t oa = part((size_t)wave * sizeof(PathRec)), ob = part((size_t)wave * sizeof(PathRec)),
+               oh = part((size_t)wave * sizeof(PtHit)), os = part((size_t)wave * 4), ol = part((size_t)total * 16),
+               oc = part(bCnt);
+  char* mem = nullptr;
+  cudaError_t e = dev_alloc(ctx, (void**)&mem, bytes, st);
+  if (e != cudaSuccess)
     return set_error(ctx, e == cudaErrorNotPermitted ? SHN_ERR_BUDGET : SHN_ERR_OOM, "path tracer state");
-  }
-  uint32_t* counters = (uint32_t*)cnt;  // [0..15] work counters, [16..31] live counts
-  int blocks = 0;
-  {
-    static int b0 = [&] { int v = 0; cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_pt_bounce<0>, kPtBlock, 0); return v; }();
-    static int b1 = [&] { int v = 0; cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_pt_bounce<1>, kPtBlock, 0); return v; }();
-    blocks = std::max(1, g->kind == SHN_GRID_UNIFORM ? b0 : b1) * ctx->num_sms;
-  }
-  if (d_stats) cudaMemsetAsync(d_stats, 0, (prm->max_depth + 1) * 4, st);
+  float4* slots = (float4*)(mem + ol);
+  PtHit* hits = (PtHit*)(mem + oh);
+  uint32_t* shadow = (uint32_t*)(mem + os);
+  PtCount* cnt = (PtCount*)(mem + oc);
+  if (d_stats) cudaMemsetAsync(d_stats, 0, ((size_t)prm->max_depth + 1) * 4, st);
   for (uint64_t g0 = 0; g0 < total; g0 += wave) {
     const uint32_t count = (uint32_t)std::min<uint64_t>(wave, total - g0);
-    PathRec* cur = (PathRec*)pa;
-    PathRec* nxt = (PathRec*)pb;
-    uint32_t* d_n = counters + 16;
-    k_pt_camera<<<(count + 255) / 256, 256, 0, st>>>(P, g0, count, cur, d_n);
+    PathRec* cur = (PathRec*)(mem + oa);
+    PathRec* nxt = (PathRec*)(mem + ob);
+    const int shade_blocks = (int)std::min<uint32_t>((count + kShadeBlock - 1) / kShadeBlock, (uint32_t)ctx->num_sms * 8u);
+    cudaMemsetAsync(cnt, 0, bCnt, st);
+    k_pt_camera<<<(count + 255) / 256, 256, 0, st>>>(P, g0, count, cur, cnt);
     for (uint32_t d = 0; d < prm->max_depth; ++d) {
-      cudaMemsetAsync(counters, 0, 4, st);
-      if (d_stats) k_add_u32<<<1, 1, 0, st>>>(d_n, d_stats + d);
-      uint32_t* d_shadow = d_stats ? d_stats + prm->max_depth : nullptr;
-      float4* slot_base = (float4*)slots;
-      if (g->kind == SHN_GRID_UNIFORM)
-        k_pt_bounce<0><<<blocks, kPtBlock, 0, st>>>(G, P, cur, d_n, d, counters, (uint32_t*)alive, slot_base, 0,
-                                                    d_shadow);
-      else
-        k_pt_bounce<1><<<blocks, kPtBlock, 0, st>>>(G, P, cur, d_n, d, counters, (uint32_t*)alive, slot_base, 0,
-                                                    d_shadow);
-      if (d + 1 < prm->max_depth) {
-        cudaMemsetAsync(status, 0, bSt, st);
-        LookbackState ls{(uint64_t*)status, (uint32_t*)((uint64_t*)status + tiles + 1), g->d_err};
-        uint32_t* d_next = d_n + 1;
-        k_pt_compact<<<(unsigned)tiles, 256, 0, st>>>(cur, (uint32_t*)alive, d_n, nxt, d_next, ls);
-        k_copy_u32<<<1, 1, 0, st>>>(d_next, d_n);
-        std::swap(cur, nxt);
-      }
+      PtCount* c = cnt + d;
+      launch_rays<false>(G, PtExtend{cur, hits}, d == 0, &c->live, &c->work0, count, ctx->num_sms, st);
+      k_pt_shade<<<shade_blocks, kShadeBlock, 0, st>>>(P, cur, hits, nxt, shadow, d, c, slots);
+      launch_rays<true>(G, PtShadow{cur, shadow, slots, P.npix}, false, &c->shadow, &c->work1, count, ctx->num_sms, st);
+      std::swap(cur, nxt);
     }
+    if (d_stats) k_pt_stats<<<1, 1, 0, st>>>(cnt, prm->max_depth, d_stats);
   }
-  k_pt_resolve<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>((const float4*)slots, (uint32_t)npix,
+  k_pt_resolve<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(slots, (uint32_t)npix,
                                                                prm->spp, d_image);
-  release();
+  dev_free(ctx, mem, bytes, st);
   e = cudaGetLastError();
   return e == cudaSuccess ? SHN_OK : cuda_status(ctx, e, "pt_render");
 }

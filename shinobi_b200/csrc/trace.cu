@@ -8,6 +8,7 @@
 #include "internal.h"
 #include "trace.cuh"
 #include "trace_coop.cuh"
+#include "rays.cuh"
 
 namespace shn {
 
@@ -107,65 +108,15 @@ __global__ void __launch_bounds__(256) k_compact_hits(const uint32_t* __restrict
       d_m);
 }
 
-struct AoParams {
-  CamView cam;
-  uint32_t image_id, spp, seed;
-  float len, offset;
-  const float4* stri;  // scene triangles, 48-byte records (v0, v1, v2)
-  uint32_t snt;
-  uint32_t npix;
-};
-
-template <int KIND, bool STATS>
-__global__ void __launch_bounds__(kTraceBlock, 6) k_trace_ao(GridView G, AoParams A,
-                                                          const uint32_t* __restrict__ ptri,
-                                                          const float* __restrict__ pt,
-                                                          const uint32_t* __restrict__ hit_idx,
-                                                          const uint32_t* d_m, uint32_t* counter,
-                                                          uint8_t* __restrict__ occ,
-                                                          unsigned long long* stats,
-                                                          uint32_t* err) {
-  const uint32_t n = (*d_m) * A.spp;
+// Any-hit rays made from the primary hits (Rays: AoRays or DiRays), spp per
+// hit pixel.
+template <int KIND, bool STATS, class Rays>
+__global__ void __launch_bounds__(kTraceBlock, 6) k_trace_from_hits(GridView G, Rays R, const uint32_t* d_m, uint32_t spp,
+                                                                 uint32_t* counter, unsigned long long* stats) {
   warp_trace<KIND, true, true>(
-      G, n, counter,
-      [&](uint32_t r, V3& o, V3& dir, float& tmax) {
-        const uint32_t k = r / A.spp, s = r - k * A.spp;
-        const uint32_t p = hit_idx[k];
-        // a compaction whose look-back gave up (error bit set) can leave a
-        // slot unwritten: such a ray becomes an empty segment, no access leaves
-        // the pixel and triangle arrays
-        const uint32_t tri = p < A.npix ? ptri[p] : kMiss;
-        if (tri >= A.snt) {
-          o = A.cam.eye;
-          dir = mk(0.f, 0.f, 1.f);
-          tmax = 0.f;
-          return;
-        }
-        const float t = pt[p];
-        const V3 d = primary_dir(A.cam, p, A.image_id);
-        const float4* rec = A.stri + 3 * (size_t)tri;
-        const V3 v0 = f4v(__ldg(rec));
-        const V3 v1 = f4v(__ldg(rec + 1));
-        const V3 v2 = f4v(__ldg(rec + 2));
-        const V3 e1 = sub(v1, v0);
-        V3 nn = normalize(cross(e1, sub(v2, v0)));
-        if (dot(nn, d) > 0.f) nn = mk(-nn.x, -nn.y, -nn.z);
-        const V3 tx = normalize(e1);
-        const V3 ty = cross(nn, tx);
-        const V3 hp = add(A.cam.eye, muls(d, t));
-        o = add(hp, muls(nn, A.offset));
-        const uint4 w = philox4x32(make_uint4(p, s, 0u, 0x414Fu), A.seed, 0u);
-        const float u1 = u01(w.x), u2 = u01(w.y);
-        float sn, cs;
-        sincos_2pi(u1, sn, cs);
-        const float rr = sqrtf(1.f - u2);
-        const float lx = sn * rr, ly = cs * rr, lz = sqrtf(u2);
-        dir = mk(tx.x * lx + ty.x * ly + nn.x * lz, tx.y * lx + ty.y * ly + nn.y * lz,
-                 tx.z * lx + ty.z * ly + nn.z * lz);
-        tmax = A.len;
-      },
+      G, (*d_m) * spp, counter, [&](uint32_t r, V3& o, V3& dir, float& tmax) { R.ray(r, o, dir, tmax); },
       [&](uint32_t r, const Hit& h, uint32_t steps, uint32_t tests) {
-        occ[r] = h.tri != kMiss ? 1 : 0;
+        R.done(r, h);
         add_counts<STATS>(stats, steps, tests);
       });
 }
@@ -189,61 +140,6 @@ __global__ void k_ao_finalize(const uint32_t* __restrict__ ptri, const uint32_t*
   uint32_t c = 0;
   for (uint32_t s = 0; s < spp; ++s) c += occ[b + s];
   ao[p] = 1.0f - (float)c / (float)spp;
-}
-
-// Direct illumination from a parallelogram light (DirectIlluminationIntegrator::shade,
-// src/Integrator/DirectIlluminationIntegrator.h:254-315, and computeDirectIllumination,
-// src/Integrator/DirectIlluminationIntegrator.h:46-168).
-struct DiParams {
-  CamView cam;
-  V3 lpos, le1, le2, lnrm, lint, ddef, bg;
-  float larea;
-  uint32_t spp, seed, image_id, nmat, npix;
-  const float4* stri;        // scene triangles, 48-byte records (v0, v1, v2)
-  const uint32_t* tri_mat;   // per scene triangle, or null
-  const float4* diffuse;     // per material, or null
-};
-
-// Shadow segment of sample s of hit pixel p: the origin is the stored hit point
-// eye + (t - EPS) d (SimpleRayBuffer::store, src/Engine/RayBuffers.h:52-55), the
-// direction runs to a uniform point of the light (AreaLightShadowRayGenerator,
-// src/Engine/RayGenerators.h:106-139; AreaLightSource::getPoint,
-// src/Primitive/LightSource.hpp:40-43); Philox replaces the KISS generator.
-SHN_D void di_segment(const DiParams& P, uint32_t p, uint32_t s, float t, V3& o, V3& L) {
-  const V3 d = primary_dir(P.cam, p, P.image_id);
-  o = add(P.cam.eye, muls(d, t - 1e-5f));
-  const uint4 w = philox4x32(make_uint4(p, s, P.image_id, 0x444Cu), P.seed, 0u);
-  const V3 lp = add(add(P.lpos, muls(P.le1, u01(w.x))), muls(P.le2, u01(w.y)));
-  L = sub(lp, o);
-}
-
-template <int KIND, bool STATS>
-__global__ void __launch_bounds__(kTraceBlock, 6) k_trace_direct(GridView G, DiParams P,
-                                                              const float* __restrict__ pt,
-                                                              const uint32_t* __restrict__ hit_idx,
-                                                              const uint32_t* d_m, uint32_t* counter,
-                                                              uint8_t* __restrict__ occ,
-                                                              unsigned long long* stats,
-                                                              uint32_t* err) {
-  const uint32_t n = (*d_m) * P.spp;
-  warp_trace<KIND, true, true>(
-      G, n, counter,
-      [&](uint32_t r, V3& o, V3& dir, float& tmax) {
-        const uint32_t k = r / P.spp, s = r - k * P.spp;
-        const uint32_t p = hit_idx[k];
-        if (p >= P.npix) {  // slot left unwritten by a look-back that gave up
-          o = P.cam.eye;
-          dir = mk(0.f, 0.f, 1.f);
-          tmax = 0.f;
-          return;
-        }
-        di_segment(P, p, s, pt[p], o, dir);
-        tmax = 0.9999f;
-      },
-      [&](uint32_t r, const Hit& h, uint32_t steps, uint32_t tests) {
-        occ[r] = h.tri != kMiss ? 1 : 0;
-        add_counts<STATS>(stats, steps, tests);
-      });
 }
 
 // Per pixel: the mean over samples of the light's contribution
@@ -310,22 +206,6 @@ int persistent_blocks(K kernel, int num_sms) {
   return std::max(1, per_sm) * num_sms;
 }
 
-GridView view_of(const shn_grid* g) {
-  GridView v;
-  v.g = g->geom;
-  v.kind = g->kind;
-  v.cells = g->cells;
-  v.leaves = g->leaves;
-  v.rv0 = g->rtri;
-  v.rv1 = g->rtri + g->num_refs;
-  v.rv2 = g->rtri + 2 * g->num_refs;
-  v.src = g->src_tri;
-  v.cbox = g->num_blocks ? (const float4*)g->cbox.ptr : nullptr;
-  v.sbox = g->num_blocks ? (const float4*)g->sbox.ptr : nullptr;
-  v.ridx = nullptr;
-  return v;
-}
-
 // Per-call scratch from the context pool, released stream-ordered.
 struct Scratch {
   shn_ctx* ctx;
@@ -349,12 +229,46 @@ struct Scratch {
   }
 };
 
+template <class Rays>
+void trace_from_hits(const shn_grid* g, const GridView& G, const Rays& R, const uint32_t* d_m, uint32_t spp,
+                     uint32_t* counter, uint32_t npix, cudaStream_t st) {
+  if (g->kind == SHN_GRID_UNIFORM && !g->stats) {
+    launch_flat_from_hits(G, R, d_m, spp, counter, (uint64_t)npix * spp, g->ctx->num_sms, st);
+    return;
+  }
+#define SHN_LAUNCH_HITS(K, S)                                                                        \
+  {                                                                                                  \
+    static int blocks = persistent_blocks(k_trace_from_hits<K, S, Rays>, g->ctx->num_sms);           \
+    k_trace_from_hits<K, S, Rays><<<blocks, kTraceBlock, 0, st>>>(G, R, d_m, spp, counter, g->stats); \
+  }
+  if (g->kind == SHN_GRID_UNIFORM) SHN_LAUNCH_HITS(0, true)
+  else if (g->stats) SHN_LAUNCH_HITS(1, true)
+  else SHN_LAUNCH_HITS(1, false)
+#undef SHN_LAUNCH_HITS
+}
+
 shn_status check_launch(shn_ctx* ctx, const char* what) {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SHN_OK : cuda_status(ctx, e, what);
 }
 
 }  // namespace
+
+GridView view_of(const shn_grid* g) {
+  GridView v;
+  v.g = g->geom;
+  v.kind = g->kind;
+  v.cells = g->cells;
+  v.leaves = g->leaves;
+  v.rv0 = g->rtri;
+  v.rv1 = g->rtri + g->num_refs;
+  v.rv2 = g->rtri + 2 * g->num_refs;
+  v.src = g->src_tri;
+  v.cbox = g->num_blocks ? (const float4*)g->cbox.ptr : nullptr;
+  v.sbox = g->num_blocks ? (const float4*)g->sbox.ptr : nullptr;
+  v.ridx = g->kind == SHN_GRID_UNIFORM ? g->indices : nullptr;
+  return v;
+}
 
 CamView make_camera(const shn_camera* c) {
   // Camera::init (src/Primitive/Camera.h:41-60), host FP32 as in the reference.
@@ -412,7 +326,9 @@ shn_status shn_trace_closest(const shn_grid* g, const shn_rays* rays, uint32_t n
                                                             g->stats, g->d_err);                          \
   }
   if (g->kind == SHN_GRID_UNIFORM) {
-    if (g->stats) SHN_LAUNCH_RAYS(0, true) else SHN_LAUNCH_RAYS(0, false)
+    if (g->stats) SHN_LAUNCH_RAYS(0, true)
+    else
+      launch_flat_closest(G, *rays, n, counter, *hits, g->ctx->num_sms, st);
   } else {
     if (g->stats) SHN_LAUNCH_RAYS(1, true) else SHN_LAUNCH_RAYS(1, false)
   }
@@ -443,7 +359,9 @@ shn_status shn_trace_any(const shn_grid* g, const shn_rays* rays, uint32_t n, ui
                                                            g->stats, g->d_err);                           \
   }
   if (g->kind == SHN_GRID_UNIFORM) {
-    if (g->stats) SHN_LAUNCH_ANY(0, true) else SHN_LAUNCH_ANY(0, false)
+    if (g->stats) SHN_LAUNCH_ANY(0, true)
+    else
+      launch_flat_any(G, *rays, n, counter, d_occluded, g->ctx->num_sms, st);
   } else {
     if (g->stats) SHN_LAUNCH_ANY(1, true) else SHN_LAUNCH_ANY(1, false)
   }
@@ -475,7 +393,9 @@ shn_status shn_trace_primary(const shn_grid* g, const shn_camera* cam, uint32_t 
                                                        g->d_err);    \
   }
   if (g->kind == SHN_GRID_UNIFORM) {
-    if (g->stats) SHN_LAUNCH_CAM(0, true) else SHN_LAUNCH_CAM(0, false)
+    if (g->stats) SHN_LAUNCH_CAM(0, true)
+    else
+      launch_flat_camera(G, C, image_id, n, counter, *hits, g->ctx->num_sms, st);
   } else {
     if (g->stats) SHN_LAUNCH_CAM(1, true) else SHN_LAUNCH_CAM(1, false)
   }
@@ -522,18 +442,7 @@ shn_status shn_trace_ao(const shn_grid* g, const shn_camera* cam, const shn_hits
   A.stri = g->src_tri;
   A.snt = g->src_nt;
   A.npix = n;
-#define SHN_LAUNCH_AO(K, S)                                                                       \
-  {                                                                                               \
-    static int blocks = persistent_blocks(k_trace_ao<K, S>, g->ctx->num_sms);                     \
-    k_trace_ao<K, S><<<blocks, kTraceBlock, 0, st>>>(G, A, primary->tri, primary->t, hit_idx, d_m, \
-                                                   counter, occ, g->stats, g->d_err);                       \
-  }
-  if (g->kind == SHN_GRID_UNIFORM) {
-    if (g->stats) SHN_LAUNCH_AO(0, true) else SHN_LAUNCH_AO(0, false)
-  } else {
-    if (g->stats) SHN_LAUNCH_AO(1, true) else SHN_LAUNCH_AO(1, false)
-  }
-#undef SHN_LAUNCH_AO
+  trace_from_hits(g, G, AoRays{A, primary->tri, primary->t, hit_idx, occ}, d_m, spp, counter, n, st);
   k_ao_finalize<<<(n + 255) / 256, 256, 0, st>>>(primary->tri, pos, occ, n, spp, d_m, d_ao, d_num_rays);
   return check_launch(g->ctx, "trace_ao");
 }
@@ -609,18 +518,7 @@ shn_status shn_shade_direct(const shn_grid* g, const shn_camera* cam, const shn_
   P.stri = g->src_tri;
   P.tri_mat = prm->tri_material;
   P.diffuse = (const float4*)prm->diffuse;
-#define SHN_LAUNCH_DI(K, S)                                                                          \
-  {                                                                                                  \
-    static int blocks = persistent_blocks(k_trace_direct<K, S>, g->ctx->num_sms);                    \
-    k_trace_direct<K, S><<<blocks, kTraceBlock, 0, st>>>(G, P, primary->t, hit_idx, d_m, counter,   \
-                                                       occ, g->stats, g->d_err);                     \
-  }
-  if (g->kind == SHN_GRID_UNIFORM) {
-    if (g->stats) SHN_LAUNCH_DI(0, true) else SHN_LAUNCH_DI(0, false)
-  } else {
-    if (g->stats) SHN_LAUNCH_DI(1, true) else SHN_LAUNCH_DI(1, false)
-  }
-#undef SHN_LAUNCH_DI
+  trace_from_hits(g, G, DiRays{P, primary->t, hit_idx, occ}, d_m, P.spp, counter, n, st);
   k_shade_direct<<<(n + 255) / 256, 256, 0, st>>>(P, primary->tri, primary->t, pos, occ, n, d_m, d_frame,
                                                   d_final, d_num_rays);
   return check_launch(g->ctx, "shade_direct");

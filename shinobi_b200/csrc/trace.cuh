@@ -1,8 +1,7 @@
-// 3D-DDA traversal of uniform and two-level grids with the watertight
-// ray/triangle test, as device functions shared by the trace, AO and
-// path-tracing kernels.
+// What the traversal engines share: the grid view, the watertight ray/triangle
+// test and camera rays.
 //
-// Traversal restates UniformGridTraverser (src/Control/Algorithm/SimpleGridTraverser.h:274-401)
+// The traversal (trace_coop.cuh, trace_flat.cuh) restates UniformGridTraverser (src/Control/Algorithm/SimpleGridTraverser.h:274-401)
 // and TwoLevelGridTraverser (src/Control/Algorithm/TwoLevelGridTraverser.h:445-671):
 // float cell coordinates, continuation while the best t exceeds the current
 // cell's exit (min of tMax), exit when a coordinate reaches res or -1 within
@@ -114,162 +113,10 @@ SHN_D bool wt_test(const RayWT& r, float4 p0, float4 p1, float4 p2, float tmin, 
 // the smaller id.
 SHN_D float next_up(float t) { return __uint_as_float(__float_as_uint(t) + 1u); }
 
-template <bool ANY>
-SHN_D bool test_range(const GridView& G, const RayWT& r, uint32_t b, uint32_t e, Hit& h) {
-  h.steps += 1;
-  const float t0 = h.t;
-  bool found = false;
-  for (uint32_t it = b; it < e; ++it) {
-    h.tests += 1;
-    const float4 p0 = __ldg(G.rv0 + it);
-    const float4 p1 = __ldg(G.rv1 + it);
-    const float4 p2 = __ldg(G.rv2 + it);
-    float t, u, v;
-    if (wt_test(r, p0, p1, p2, kEps, found ? next_up(h.t) : t0, t, u, v)) {
-      const uint32_t id = __float_as_uint(p0.w);
-      if (!found || t < h.t || id < h.tri) {
-        h.t = t;
-        h.tri = id;
-        h.u = u;
-        h.v = v;
-        found = true;
-      }
-      if (ANY) return true;
-    }
-  }
-  return false;
-}
-
 SHN_D int min_dim(V3 t) { return (t.x < t.y) ? ((t.x < t.z) ? 0 : 2) : ((t.y < t.z) ? 1 : 2); }
 SHN_D float clampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 SHN_D void bump(V3& v, int d, float a) {
   if (d == 0) v.x += a; else if (d == 1) v.y += a; else v.z += a;
-}
-
-template <bool ANY>
-SHN_D void trace_uniform(const GridView& G, V3 org, V3 dir, Hit& h) {
-  const Geom& g = G.g;
-  const V3 rcp = divv(mk(1.f, 1.f, 1.f), dir);
-  const RayWT w = wt_setup(org, dir);
-  if (!(h.t > 0.f)) return;
-  const V3 t1 = mul(sub(g.gmin, org), rcp);
-  V3 t2 = mul(sub(g.gmax, org), rcp);
-  const V3 tmn = vmin(t1, t2);
-  t2 = vmax(t1, t2);
-  const float tEntry = fmaxf(fmaxf(tmn.x, tmn.y), tmn.z);
-  const float tExit = fminf(fminf(t2.x, t2.y), t2.z);
-  if (tExit <= tEntry || tExit < 0.f) return;
-  const float te = tEntry + kEps;
-  const V3 entry = (tEntry >= 0.f) ? add(org, divv(mk(te, te, te), rcp)) : org;
-  V3 cell = mul(sub(entry, g.gmin), g.rcpTrav);
-  cell = mk(floorf(cell.x), floorf(cell.y), floorf(cell.z));
-  const V3 tmp = mk(rcp.x > 0.f ? 1.f : 0.f, rcp.y > 0.f ? 1.f : 0.f, rcp.z > 0.f ? 1.f : 0.f);
-  V3 tMax = mul(sub(add(mul(add(cell, tmp), g.cs), g.gmin), org), rcp);
-  bool valid = (cell.x != (rcp.x > 0.f ? g.resf.x : -1.f)) && (cell.y != (rcp.y > 0.f ? g.resf.y : -1.f)) &&
-               (cell.z != (rcp.z > 0.f ? g.resf.z : -1.f));
-  const int cap = g.res[0] + g.res[1] + g.res[2] + 3;
-  // An empty cell of a large uniform grid holds [D, D), D its distance to the
-  // nearest non-empty cell: the next D - 1 cells are empty and are stepped
-  // through without fetching (counted as visits all the same).
-  uint32_t skip = 0;
-  for (int step = 0; valid && step < cap; ++step) {
-    if (skip == 0) {
-      const uint32_t cx = (uint32_t)clampf(cell.x, 0.f, g.resf.x - 1.f);
-      const uint32_t cy = (uint32_t)clampf(cell.y, 0.f, g.resf.y - 1.f);
-      const uint32_t cz = (uint32_t)clampf(cell.z, 0.f, g.resf.z - 1.f);
-      const uint2 range = __ldg(G.cells + (cx + cy * (uint32_t)g.res[0] + cz * (uint32_t)g.res[0] * (uint32_t)g.res[1]));
-      if (test_range<ANY>(G, w, range.x, range.y, h)) return;
-      if (range.y <= range.x && range.x > 0u) skip = range.x - 1u;
-    } else {
-      --skip;
-      h.steps += 1;
-    }
-    valid = h.t > tMax.x || h.t > tMax.y || h.t > tMax.z;
-    if (!valid) break;
-    const int d = min_dim(tMax);
-    const float rd = sel(d, rcp);
-    bump(cell, d, rd > 0.f ? 1.f : -1.f);
-    bump(tMax, d, sel(d, g.cs) * fabsf(rd));
-    const float cd = sel(d, cell);
-    valid = !(fabsf(cd - sel(d, g.resf)) < 0.1f || fabsf(cd + 1.f) < 0.1f);
-  }
-}
-
-template <bool ANY>
-SHN_D void trace_two_level(const GridView& G, V3 org, V3 dir, Hit& h) {
-  const Geom& g = G.g;
-  const V3 rcp = divv(mk(1.f, 1.f, 1.f), dir);
-  const RayWT w = wt_setup(org, dir);
-  if (!(h.t > 0.f)) return;
-  const V3 t1 = mul(sub(g.gmin, org), rcp);
-  V3 t2 = mul(sub(g.gmax, org), rcp);
-  const V3 tmn = vmin(t1, t2);
-  t2 = vmax(t1, t2);
-  float tEntry = fmaxf(fmaxf(tmn.x, tmn.y), tmn.z);
-  const float tExit = fminf(fminf(t2.x, t2.y), t2.z);
-  if (tExit <= tEntry || tExit < 0.f) return;
-  tEntry = fmaxf(0.f, tEntry);
-  const float te = tEntry + kEps;
-  const V3 entry = add(org, divv(mk(te, te, te), rcp));
-  V3 cell = mul(sub(entry, g.gmin), g.rcpTrav);
-  cell = mk(floorf(cell.x), floorf(cell.y), floorf(cell.z));
-  const V3 tmp = mk(rcp.x > 0.f ? 1.f : 0.f, rcp.y > 0.f ? 1.f : 0.f, rcp.z > 0.f ? 1.f : 0.f);
-  V3 tMax = mul(sub(add(mul(add(cell, tmp), g.cs), g.gmin), org), rcp);
-  bool valid = (cell.x != (rcp.x > 0.f ? g.resf.x : -1.f)) && (cell.y != (rcp.y > 0.f ? g.resf.y : -1.f)) &&
-               (cell.z != (rcp.z > 0.f ? g.resf.z : -1.f));
-  const int cap = g.res[0] + g.res[1] + g.res[2] + 3;
-  for (int step = 0; valid && step < cap; ++step) {
-    const uint32_t cx = (uint32_t)clampf(cell.x, 0.f, g.resf.x - 1.f);
-    const uint32_t cy = (uint32_t)clampf(cell.y, 0.f, g.resf.y - 1.f);
-    const uint32_t cz = (uint32_t)clampf(cell.z, 0.f, g.resf.z - 1.f);
-    const uint2 cw = __ldg(G.cells + (cx + cy * (uint32_t)g.res[0] + cz * (uint32_t)g.res[0] * (uint32_t)g.res[1]));
-    if (cw.y & kNotEmpty) {
-      const V3 ent = add(org, divv(mk(tEntry, tEntry, tEntry), rcp));
-      const V3 cres = mk((float)(cw.y & 0xFFu), (float)((cw.y >> 8) & 0xFFu), (float)((cw.y >> 16) & 0xFFu));
-      const V3 subRCP = mul(g.rcpTrav, cres);
-      const V3 minB = add(mul(cell, g.cs), g.gmin);
-      V3 sc;
-      sc.x = floorf((ent.x - minB.x) * subRCP.x);
-      sc.y = floorf((ent.y - minB.y) * subRCP.y);
-      sc.z = floorf((ent.z - minB.z) * subRCP.z);
-      const V3 scs = divv(mk(1.f, 1.f, 1.f), subRCP);
-      sc = vmin(sub(cres, mk(1.f, 1.f, 1.f)), vmax(sc, mk(0.f, 0.f, 0.f)));
-      V3 sMax;
-      sMax.x = ((sc.x + tmp.x) * scs.x + minB.x - org.x) * rcp.x;
-      sMax.y = ((sc.y + tmp.y) * scs.y + minB.y - org.y) * rcp.y;
-      sMax.z = ((sc.z + tmp.z) * scs.z + minB.z - org.z) * rcp.z;
-      bool v2 = true;
-      const int cap2 = (int)cres.x + (int)cres.y + (int)cres.z + 3;
-      for (int s2 = 0; v2 && s2 < cap2; ++s2) {
-        const uint32_t li = cw.x + (uint32_t)(sc.x + cres.x * sc.y + cres.x * cres.y * sc.z);
-        const uint2 range = __ldg(G.leaves + li);
-        if (test_range<ANY>(G, w, range.x, range.y, h)) return;
-        v2 = h.t > sMax.x || h.t > sMax.y || h.t > sMax.z;
-        if (!v2) break;
-        const int d = min_dim(sMax);
-        const float rd = sel(d, rcp);
-        bump(sc, d, rd > 0.f ? 1.f : -1.f);
-        bump(sMax, d, sel(d, scs) * fabsf(rd));
-        const float cd = sel(d, sc);
-        v2 = !(fabsf(cd - sel(d, cres)) < 0.1f || fabsf(cd + 1.f) < 0.1f);
-      }
-    }
-    valid = h.t > tMax.x || h.t > tMax.y || h.t > tMax.z;
-    if (!valid) break;
-    const int d = min_dim(tMax);
-    tEntry = sel(d, tMax);
-    const float rd = sel(d, rcp);
-    bump(cell, d, rd > 0.f ? 1.f : -1.f);
-    bump(tMax, d, sel(d, g.cs) * fabsf(rd));
-    const float cd = sel(d, cell);
-    valid = !(fabsf(cd - sel(d, g.resf)) < 0.1f || fabsf(cd + 1.f) < 0.1f);
-  }
-}
-
-template <int KIND, bool ANY>
-SHN_D void trace_ray(const GridView& G, V3 org, V3 dir, Hit& h) {
-  if (KIND == 0) trace_uniform<ANY>(G, org, dir, h);
-  else trace_two_level<ANY>(G, org, dir, h);
 }
 
 // Camera::init result + RegularPixelSampler<1,1> (src/Primitive/Camera.h:67-70,

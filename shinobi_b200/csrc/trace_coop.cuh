@@ -19,7 +19,7 @@
 // a warp of 32 once all lanes are done (PACKET).
 //
 // The per-ray sequence of cell visits, tests and continuation decisions is
-// exactly that of trace_uniform / trace_two_level (trace.cuh) (block culling
+// that of the reference's traversers (block culling
 // and the empty-leaf skips only leave out work that cannot change the result);
 // the closest hit of a range is the least (t, triangle id) of its candidates,
 // the winner the reference's strict-< loop keeps over references in (cell,
@@ -406,7 +406,7 @@ SHN_D bool wt_test_p(V3 org, float Sx, float Sy, float Sz, float4 p0, float4 p1,
 // Closest: returns the packed argmin key (t bits << 32 | triangle id) in every
 // lane, or ~0 when nothing beats tbest.  Any: returns a hit's key or ~0.  A
 // lane's candidate must beat tbest strictly and may tie the lane's running
-// minimum (the least (t, id) wins, as in test_range).
+// minimum (the least (t, id) wins).
 // L2 latency is covered by the other resident warps: the kernels that run
 // this engine are limited to 64 registers (8 blocks of 128 threads per SM),
 // which measured faster than staging the next chunk in registers or in

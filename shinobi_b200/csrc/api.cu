@@ -95,19 +95,22 @@ __global__ void k_lerp_vertices(const float* __restrict__ kf1, const float* __re
     out[i] = i < m ? __ldg(kf1 + i) * omc + __ldg(kf2 + i) * c : __ldg(kf2 + i);
 }
 
-shn_status refresh_bounds(shn_scene* s, cudaStream_t st) {
-  float* d6 = nullptr;
+// The triangle records and the bounds of the scene's vertices.
+shn_status pack_scene(shn_scene* s, cudaStream_t st) {
+  uint32_t* d6 = nullptr;
   cudaError_t e = dev_alloc(s->ctx, (void**)&d6, 64, st);
   if (e != cudaSuccess) return alloc_status(s->ctx, e, "bounds");
-  launch_bounds_reduce(s->tri, s->nt, d6, st);
-  float h6[6];
+  launch_pack_triangles(s->vtx, s->idx, s->nt, s->tri, d6, st);
+  uint32_t h6[6];
   cudaMemcpyAsync(h6, d6, sizeof(h6), cudaMemcpyDeviceToHost, st);
   dev_free(s->ctx, d6, 64, st);
   e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_status(s->ctx, e, "scene bounds");
+  float b[6];
+  for (int i = 0; i < 6; ++i) b[i] = bounds_value(h6[i]);
   for (int i = 0; i < 3; ++i)
-    if (!(h6[i] <= h6[i + 3]) && s->nt) return set_error(s->ctx, SHN_ERR_INVALID, "empty or non-finite scene bounds");
-  memcpy(s->bounds, h6, sizeof(h6));
+    if (!(b[i] <= b[i + 3]) && s->nt) return set_error(s->ctx, SHN_ERR_INVALID, "empty or non-finite scene bounds");
+  memcpy(s->bounds, b, sizeof(b));
   return SHN_OK;
 }
 
@@ -177,8 +180,7 @@ shn_status scene_reload(shn_scene* s, const float* vtx, uint32_t nv, const uint3
   if (nv) rc = copy_in(ctx, s->vtx, vtx, 12 * (size_t)nv, SHN_MEM_HOST, st);
   if (!rc && nt) rc = copy_in(ctx, s->idx, idx, 12 * (size_t)nt, SHN_MEM_HOST, st);
   if (rc) return rc;
-  launch_pack_triangles(s->vtx, s->idx, nt, s->tri, st);
-  return refresh_bounds(s, st);
+  return pack_scene(s, st);
 }
 }  // namespace shn
 
@@ -279,8 +281,7 @@ shn_status shn_scene_create(shn_ctx* ctx, const float* vtx, uint32_t nv, const u
   if (nv) rc = copy_in(ctx, s->vtx, vtx, 12 * (size_t)nv, mem, st);
   if (!rc && nt) rc = copy_in(ctx, s->idx, idx, 12 * (size_t)nt, mem, st);
   if (!rc) {
-    launch_pack_triangles(s->vtx, s->idx, nt, s->tri, st);
-    rc = refresh_bounds(s, st);
+    rc = pack_scene(s, st);
   }
   if (rc) {
     shn_scene_destroy(s);
@@ -331,8 +332,7 @@ shn_status shn_scene_update_vertices(shn_scene* s, const float* vtx, uint32_t nv
     rc = copy_in(s->ctx, s->vtx, vtx, 12 * (size_t)nv, mem, st);
     if (rc) return rc;
   }
-  launch_pack_triangles(s->vtx, s->idx, s->nt, s->tri, st);
-  return refresh_bounds(s, st);
+  return pack_scene(s, st);
 }
 
 shn_status shn_scene_interpolate_vertices(shn_scene* s, const float* kf1, uint32_t n1, const float* kf2,
@@ -346,8 +346,7 @@ shn_status shn_scene_interpolate_vertices(shn_scene* s, const float* kf1, uint32
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_status(s->ctx, e, "interpolate vertices");
   }
-  launch_pack_triangles(s->vtx, s->idx, s->nt, s->tri, st);
-  return refresh_bounds(s, st);
+  return pack_scene(s, st);
 }
 
 shn_status shn_scene_bounds(const shn_scene* s, float out[6]) {

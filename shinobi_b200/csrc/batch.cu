@@ -237,7 +237,7 @@ void enqueue_build(shn_batch* b, cudaStream_t st) {
   // references each and the trace reads a reference's triangle through its
   // id (indices[]), which measured cheaper than gathering and writing 96 bytes
   // per reference in the build; the ranges are written by tiles of cells
-  launch_cell_ranges(b->sorted, b->P, b->total_cells, b->cells, b->indices, st);
+  launch_cell_ranges(b->sorted, b->P, b->total_cells, b->cells, b->indices, 0u, st);
 }
 
 GridView batch_view(const shn_batch* b) {

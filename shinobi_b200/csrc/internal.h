@@ -72,7 +72,7 @@ struct shn_grid {
   uint2* cells = nullptr;       // uniform ranges / two-level cell words
   uint2* leaves = nullptr;      // two-level leaf ranges
   uint32_t* indices = nullptr;  // tri id per reference
-  float4* rtri = nullptr;       // 3*num_refs: reference-ordered v0[], v1[], v2[]
+  float4* rtri = nullptr;       // two-level: 3*num_refs: reference-ordered v0[], v1[], v2[]
   uint64_t* top_pairs = nullptr;  // two-level: sorted top pairs; uniform: sorted pairs
   // two-level grids: the build runs on the triangles in Morton order (perm_tri,
   // w = original id), so the pairs' low words are positions in that order;
@@ -156,9 +156,11 @@ float grid_build_ms(const shn_grid* g);
 // resolutions res[3*i..3*i+2] over nt 48-byte triangle records; synchronous.
 shn_status sah_refs_list(shn_ctx* ctx, const float4* tri, uint32_t nt, const float b[6], const int32_t* res,
                          uint32_t k, uint64_t* refs, float* cost, cudaStream_t st);
-void launch_pack_triangles(const float* vtx, const uint32_t* idx, uint32_t nt, float4* tri,
+// Packs the records and leaves the vertex bounds in d_key6 as ordered keys
+// (min x, y, z, max x, y, z; bounds_value decodes one).
+void launch_pack_triangles(const float* vtx, const uint32_t* idx, uint32_t nt, float4* tri, uint32_t* d_key6,
                            cudaStream_t st);
-void launch_bounds_reduce(const float4* tri, uint32_t nt, float* d_out6, cudaStream_t st);
+float bounds_value(uint32_t key);
 
 // batched multi-scene build (build.cu)
 struct BatchScene {
@@ -179,10 +181,9 @@ void launch_batch_emit(const float4* tri, uint32_t T, const uint32_t* tri_off, c
                        uint32_t* err, uint32_t* hist, SortPlan hplan, cudaStream_t st);
 // Ranges of all C cells (empty ones (0, 0)) and indices[], written by tiles
 // of cells: needs no cleared cell array.
-void launch_cell_ranges(const uint64_t* keys, uint32_t n, uint64_t C, uint2* ranges, uint32_t* indices,
+// (key's triangle + id0)
+void launch_cell_ranges(const uint64_t* keys, uint32_t n, uint64_t C, uint2* ranges, uint32_t* indices, uint32_t id0,
                         cudaStream_t st);
-void launch_ranges(const uint64_t* keys, uint32_t n, uint2* ranges, uint32_t* indices,
-                   const float4* tri, uint32_t T, float4* rtri, cudaStream_t st);
 
 // trace.cu
 struct CamView;

@@ -41,12 +41,12 @@ struct ServeSeg {
 };
 
 struct ServeAcc {
-  static constexpr bool kIndirect = false;
+  static constexpr bool kIndirect = true;  // uniform grids: triangles through indices[]
   const ServeSeg* __restrict__ segs;
   SHN_D const Geom& geom(uint32_t s) const { return segs[s].g.g; }
   SHN_D const uint2* cells(uint32_t s) const { return segs[s].g.cells; }
   SHN_D const uint2* leaves(uint32_t s) const { return segs[s].g.leaves; }
-  SHN_D Refs refs(uint32_t s) const { return Refs{segs[s].g.rv0, segs[s].g.rv1, segs[s].g.rv2}; }
+  SHN_D Refs refs(uint32_t s) const { return refs_of(segs[s].g); }
 };
 
 // Rays are AoS records of 8 floats: ox, oy, oz, dx, dy, dz, tmax, unused.
@@ -366,17 +366,7 @@ void issue_launch(shn_server* s, ServeLaunch& la, int slot_index, std::unique_lo
     ServeSeg& sg = la.h_segs[k];
     sg.ray_begin = la.begin[k];
     sg.anyhit = r->r.kind == SHN_REQ_ANY ? 1u : 0u;
-    sg.g.g = g->geom;
-    sg.g.kind = g->kind;
-    sg.g.cells = g->cells;
-    sg.g.leaves = g->leaves;
-    sg.g.rv0 = g->rtri;
-    sg.g.rv1 = g->rtri + g->num_refs;
-    sg.g.rv2 = g->rtri + 2 * g->num_refs;
-    sg.g.src = g->src_tri;
-    sg.g.cbox = g->num_blocks ? (const float4*)g->cbox.ptr : nullptr;
-    sg.g.sbox = g->num_blocks ? (const float4*)g->sbox.ptr : nullptr;
-    sg.g.ridx = nullptr;
+    sg.g = view_of(g);
   }
   s->max_requests_per_launch = std::max<uint64_t>(s->max_requests_per_launch, la.reqs.size());
   la.busy = true;

@@ -255,18 +255,21 @@ shn_status check_launch(shn_ctx* ctx, const char* what) {
 }  // namespace
 
 GridView view_of(const shn_grid* g) {
-  GridView v;
+  GridView v{};
   v.g = g->geom;
   v.kind = g->kind;
   v.cells = g->cells;
   v.leaves = g->leaves;
-  v.rv0 = g->rtri;
-  v.rv1 = g->rtri + g->num_refs;
-  v.rv2 = g->rtri + 2 * g->num_refs;
   v.src = g->src_tri;
-  v.cbox = g->num_blocks ? (const float4*)g->cbox.ptr : nullptr;
-  v.sbox = g->num_blocks ? (const float4*)g->sbox.ptr : nullptr;
-  v.ridx = g->kind == SHN_GRID_UNIFORM ? g->indices : nullptr;
+  if (g->kind == SHN_GRID_UNIFORM) {
+    v.ridx = g->indices;
+  } else {
+    v.rv0 = g->rtri;
+    v.rv1 = g->rtri + g->num_refs;
+    v.rv2 = g->rtri + 2 * g->num_refs;
+    v.cbox = g->num_blocks ? (const float4*)g->cbox.ptr : nullptr;
+    v.sbox = g->num_blocks ? (const float4*)g->sbox.ptr : nullptr;
+  }
   return v;
 }
 

@@ -9,9 +9,10 @@
 // each DDA level carries a step cap of res.x+res.y+res.z+3.  Any-hit stops at
 // the first hit in (EPS, tmax).
 //
-// Triangles are read from the grid's reference-ordered SoA float4 copy
-// (v0[ref], v1[ref], v2[ref]; v0.w carries the triangle id), so a cell's
-// candidates are contiguous and no indices[] indirection is needed.
+// Two-level grids keep a reference-ordered SoA float4 copy of the triangles
+// (v0[ref], v1[ref], v2[ref]; v0.w carries the triangle id), so a leaf's
+// candidates are contiguous; uniform grids read the scene's records through
+// indices[].
 #pragma once
 #include "common.cuh"
 

@@ -1010,9 +1010,11 @@ SHN_D void warp_trace_acc(const Acc& acc, uint32_t n, uint32_t* counter, Src&& s
   }
 }
 
-// Grid access of a lane: the single-grid kernels use one GridView for every lane.
+// Grid access of a lane: the single-grid kernels use one GridView for every
+// lane.  Uniform grids (KIND 0) have no reference-ordered copy.
+template <int KIND>
 struct OneGrid {
-  static constexpr bool kIndirect = false;
+  static constexpr bool kIndirect = KIND == 0;
   const GridView* G;
   SHN_D const Geom& geom(uint32_t) const { return G->g; }
   SHN_D const uint2* cells(uint32_t) const { return G->cells; }
@@ -1022,8 +1024,8 @@ struct OneGrid {
 
 template <int KIND, bool ANY, bool PACKET = false, class Src, class Sink>
 SHN_D void warp_trace(const GridView& G, uint32_t n, uint32_t* counter, Src&& src, Sink&& sink) {
-  warp_trace_acc<KIND, ANY, true, PACKET>(
-      OneGrid{&G}, n, counter,
+  warp_trace_acc<KIND, ANY, KIND == 1, PACKET>(
+      OneGrid<KIND>{&G}, n, counter,
       [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t& scene, uint32_t&) {
         scene = 0;
         src(i, o, d, tmax);

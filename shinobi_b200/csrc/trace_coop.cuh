@@ -519,7 +519,15 @@ SHN_D uint64_t warp_range_cull_p(const Refs& G, V3 org, V3 cr, float Sx, float S
   const uint32_t kb = b >> 5, ke = (e - 1) >> 5;
   uint32_t ntest = 0;
   bool done = false;
-  for (uint32_t s = kb >> 5; s <= (ke >> 5) && !done; ++s) {
+  for (uint32_t s0 = kb >> 5; s0 <= (ke >> 5) && !done; s0 += 32u) {
+  // the super-blocks the ray meets, one box per lane
+  const uint32_t sl = min(s0 + lane, ke >> 5);
+  uint32_t cand = __ballot_sync(0xFFFFFFFFu, s0 + lane <= (ke >> 5) &&
+                                                 box_meets(org, cr, __ldg(G.sbox + 2 * (size_t)sl),
+                                                           __ldg(G.sbox + 2 * (size_t)sl + 1), tbest));
+  while (cand && !done) {
+    const uint32_t s = s0 + (uint32_t)(__ffs(cand) - 1);
+    cand &= cand - 1;
     uint64_t wk = key;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -527,7 +535,8 @@ SHN_D uint64_t warp_range_cull_p(const Refs& G, V3 org, V3 cr, float Sx, float S
       wk = other < wk ? other : wk;
     }
     const float tw = wk == ~0ull ? tbest : __uint_as_float((uint32_t)(wk >> 32));
-    if (!box_meets(org, cr, __ldg(G.sbox + 2 * (size_t)s), __ldg(G.sbox + 2 * (size_t)s + 1), tw)) continue;
+    if (!ANY && tw < tbest && !box_meets(org, cr, __ldg(G.sbox + 2 * (size_t)s), __ldg(G.sbox + 2 * (size_t)s + 1), tw))
+      continue;
     const uint32_t k = 32u * s + lane;
     const bool need = k >= kb && k <= ke &&
                       box_meets(org, cr, __ldg(G.cbox + 2 * (size_t)k), __ldg(G.cbox + 2 * (size_t)k + 1), tw);
@@ -572,6 +581,7 @@ SHN_D uint64_t warp_range_cull_p(const Refs& G, V3 org, V3 cr, float Sx, float S
         break;
       }
     }
+  }
   }
   tests += ntest;
 #pragma unroll
@@ -713,7 +723,26 @@ SHN_D void group_cull_p(const Refs& G, const LaneG* park, unsigned long long* gk
   const V3 mycr = cull_rcp(park[lane].rcp);
   const float mytb0 = park[lane].tbest;
   uint32_t mycount = 0;
-  for (uint32_t s = kb >> 5; s <= (ke >> 5) && live; ++s) {
+  for (uint32_t s0 = kb >> 5; s0 <= (ke >> 5) && live; s0 += 32u) {
+  // A few rays: the super-blocks any of them meets, one box per lane, ray by
+  // ray (one step per ray for 32 boxes); many rays: one step per box for all
+  // rays, below, costs less.
+  uint32_t cand = (ke >> 5) - s0 >= 31u ? 0xFFFFFFFFu : (2u << ((ke >> 5) - s0)) - 1u;
+  if (__popc(live) < __popc(cand)) {
+    const uint32_t sl = min(s0 + lane, ke >> 5);
+    const float4 smn = __ldg(G.sbox + 2 * (size_t)sl), smx = __ldg(G.sbox + 2 * (size_t)sl + 1);
+    bool met = false;
+    for (uint32_t m = live; m; m &= m - 1) {
+      const int r = __ffs(m) - 1;
+      const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + r);
+      const float tb = k == ~0ull ? park[r].tbest : __uint_as_float((uint32_t)(k >> 32));
+      met = met || box_meets(park[r].org, cull_rcp(park[r].rcp), smn, smx, tb);
+    }
+    cand &= __ballot_sync(0xFFFFFFFFu, met);
+  }
+  while (cand && live) {
+    const uint32_t s = s0 + (uint32_t)(__ffs(cand) - 1);
+    cand &= cand - 1;
     bool in = false;
     if (mine && ((live >> lane) & 1u)) {
       const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + lane);
@@ -740,9 +769,21 @@ SHN_D void group_cull_p(const Refs& G, const LaneG* park, unsigned long long* gk
     while (U && live) {
       const int bl = __ffs(U) - 1;
       U &= U - 1;
-      const uint32_t rays = __shfl_sync(0xFFFFFFFFu, need, bl) & live;
+      uint32_t rays = __shfl_sync(0xFFFFFFFFu, need, bl) & live;
       if (!rays) continue;
       const uint32_t kk = 32u * s + (uint32_t)bl;
+      if (!ANY) {
+        // the bounds may have shrunk since: each lane looks at its own ray again
+        // (a step per block against a step per ray and block)
+        bool still = false;
+        if ((rays >> lane) & 1u) {
+          const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + lane);
+          still = k == ~0ull || box_meets(myo, mycr, __ldg(G.cbox + 2 * (size_t)kk), __ldg(G.cbox + 2 * (size_t)kk + 1),
+                                          __uint_as_float((uint32_t)(k >> 32)));
+        }
+        rays = __ballot_sync(0xFFFFFFFFu, still);
+        if (!rays) continue;
+      }
       if ((rays >> lane) & 1u) mycount += block_refs(kk, b, e);
       const uint32_t it = 32u * kk + lane;
       const bool ok = it >= b && it < e;
@@ -775,6 +816,7 @@ SHN_D void group_cull_p(const Refs& G, const LaneG* park, unsigned long long* gk
         }
       }
     }
+  }
   }
   if (mine) gend[lane] = b + mycount;
   __syncwarp();

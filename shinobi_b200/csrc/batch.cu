@@ -42,6 +42,7 @@ struct shn_batch {
   uint32_t* h_pinned = nullptr;
   uint64_t total_cells = 0;
   uint32_t P = 0;                      // planned pair count
+  bool keep_rows = false;              // the rows of the count fit the second key buffer
   shn::SortPlan plan{0, 8, 0};             // digit plan of the sort over the global cell bits
   uint64_t* sorted = nullptr;
   bool planned = false, built = false;
@@ -205,13 +206,18 @@ shn_status plan(shn_batch* b, cudaStream_t st) {
   if (e != cudaSuccess) return alloc_err(b, e, "batch plan");
   cudaMemcpyAsync(b->d_scenes, b->scenes.data(), sizeof(BatchScene) * b->ns, cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(b->d_err, 0, 64, st);
-  launch_batch_count(b->tri, b->T, b->d_tri_off, b->d_scenes, b->ns, b->scan_ws, b->d_err, b->offs, st);
+  launch_batch_count(b->tri, b->T, b->d_tri_off, b->d_scenes, b->ns, b->scan_ws, nullptr, 0, b->d_err, b->offs, st);
+  b->h_pinned[4] = b->h_pinned[5] = 0;
+  if (b->T) cudaMemcpyAsync(b->h_pinned + 4, batch_row_count(b->scan_ws, b->T), 8, cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(b->h_pinned, b->offs + b->T, 4, cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(b->h_pinned + 1, b->d_err, 4, cudaMemcpyDeviceToHost, st);
   e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_status(b->ctx, e, "batch plan");
   if (b->h_pinned[1]) return set_error(b->ctx, SHN_ERR_TIMEOUT, "bounded device wait gave up (batch plan)");
   b->P = b->h_pinned[0];
+  // the emission reads the rows that the count kept in the second key buffer,
+  // if all of them fit there
+  b->keep_rows = (b->h_pinned[4] | (uint64_t)b->h_pinned[5] << 32) <= b->P;
   if (b->P >= (1u << 30)) return set_error(b->ctx, SHN_ERR_INVALID, "more than 2^30 cell references in the batch");
   b->plan = sort_plan(key_bits_for(co ? co - 1 : 0));
   e = own(b, (void**)&b->keys[0], (size_t)b->P * 8, st);
@@ -227,9 +233,10 @@ shn_status plan(shn_batch* b, cudaStream_t st) {
 // The build as a sequence of launches with fixed sizes (no host sync): capturable.
 void enqueue_build(shn_batch* b, cudaStream_t st) {
   cudaMemsetAsync(b->d_err, 0, 4, st);
-  launch_batch_count(b->tri, b->T, b->d_tri_off, b->d_scenes, b->ns, b->scan_ws, b->d_err, b->offs, st);
+  uint64_t* rows = b->keep_rows ? b->keys[1] : nullptr;
+  launch_batch_count(b->tri, b->T, b->d_tri_off, b->d_scenes, b->ns, b->scan_ws, rows, b->P, b->d_err, b->offs, st);
   sort_prepare(b->sort_ws, st);
-  launch_batch_emit(b->tri, b->T, b->d_tri_off, b->d_scenes, b->ns, b->offs, b->keys[0], b->P, b->d_err,
+  launch_batch_emit(b->tri, b->T, b->d_tri_off, b->d_scenes, b->ns, b->offs, b->scan_ws, rows, b->keys[0], b->P, b->d_err,
                     sort_hist_counts(b->sort_ws), b->plan, st);
   b->sorted = onesweep_sort(b->keys[0], b->keys[1], b->P, 32, b->plan, b->sort_ws, b->d_err, st, true,
                             b->sort_tile);

@@ -171,9 +171,15 @@ SHN_D void leaf_unit(V3 a, V3 b, V3 c, const Geom& g, uint32_t topCell, uint32_t
 }
 
 // ---- unit makers: item index -> unit ------------------------------------------------
+// item(i, id, stride): the item's key word and cell strides, as its unit has them
 struct TopMaker {
   TriArr tri;
   Geom g;
+  SHN_D void item(uint32_t t, uint32_t& id, uint32_t stride[2]) const {
+    id = t;
+    stride[0] = (uint32_t)g.resf.x;
+    stride[1] = (uint32_t)(g.resf.x * g.resf.y);
+  }
   SHN_D bool operator()(uint32_t t, Unit& U) const {
     V3 a, b, c;
     load_tri(tri, t, a, b, c);
@@ -187,6 +193,13 @@ struct LeafMaker {
   const uint64_t* top;  // sorted (top cell << 32 | tri)
   const uint2* cells;   // top cell words
   Geom g;
+  SHN_D void item(uint32_t i, uint32_t& id, uint32_t stride[2]) const {
+    const uint64_t k = top[i];
+    const uint32_t y = cells[(uint32_t)(k >> 32)].y;
+    id = (uint32_t)k;
+    stride[0] = y & 0xFFu;
+    stride[1] = (y & 0xFFu) * ((y >> 8) & 0xFFu);
+  }
   SHN_D bool operator()(uint32_t i, Unit& U) const {
     const uint64_t k = top[i];
     const uint32_t c = (uint32_t)(k >> 32), t = (uint32_t)k;
@@ -207,7 +220,7 @@ constexpr int kUnitWarps = kScanBlock / 32;
 // most of its time waiting at the tile barrier).
 template <class Maker>
 __global__ void __launch_bounds__(kScanBlock) k_count_groups(Maker mk, uint32_t n, uint32_t* __restrict__ counts,
-                                                            uint32_t* group_counter) {
+                                                            uint32_t* group_counter, RowStore S) {
   __shared__ Unit su[kUnitWarps][32];
   __shared__ uint32_t acc[kUnitWarps][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -220,7 +233,7 @@ __global__ void __launch_bounds__(kScanBlock) k_count_groups(Maker mk, uint32_t 
     const uint32_t i = gidx * 32u + lane;
     const bool valid = i < n && mk(i, su[warp][lane]);
     __syncwarp();
-    const uint32_t c = warp_count_units(su[warp], acc[warp], valid);
+    const uint32_t c = warp_count_units(su[warp], acc[warp], valid, S, gidx);
     if (i < n) counts[i] = c;
     __syncwarp();
   }
@@ -235,35 +248,71 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_inplace(uint32_t* data, uin
 }
 
 // Keys of every item at offs[item]: 32 items per warp step, coalesced stores.
-// hist (optional): the sort's digit counts ([pass][512]) of the keys' cell
-// bits under the sort plan hp, counted here so that the sort needs no
-// histogram pass over the keys.
+// hist: the sort's digit counts ([pass][512]) of the keys' cell bits under the
+// sort plan hp, counted here so that the sort needs no histogram pass over the
+// keys.  groups (optional): only the groups whose rows were not kept.
 template <class Maker>
 __global__ void __launch_bounds__(kScanBlock) k_emit_units(Maker mk, uint32_t n,
                                                           const uint32_t* __restrict__ offs,
                                                           uint64_t* __restrict__ keys, uint32_t cap,
-                                                          uint32_t* err, uint32_t* hist, SortPlan hp) {
+                                                          uint32_t* err, uint32_t* hist, SortPlan hp,
+                                                          const uint2* __restrict__ gtab) {
   __shared__ Unit su[kUnitWarps][32];
   __shared__ uint32_t shist[4 * 512];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (hist) {
-    for (int i = threadIdx.x; i < 4 * 512; i += kScanBlock) shist[i] = 0u;
-    __syncthreads();
-  }
+  for (int i = threadIdx.x; i < 4 * 512; i += kScanBlock) shist[i] = 0u;
+  __syncthreads();
   const uint32_t groups = (n + 31u) / 32u;
   for (uint32_t gi = blockIdx.x * kUnitWarps + warp; gi < groups; gi += gridDim.x * kUnitWarps) {
+    if (gtab && gtab[gi].x != kNoRows) continue;
     const uint32_t i = gi * 32u + lane;
     const bool valid = i < n && mk(i, su[warp][lane]);
     const uint32_t out = offs[gi * 32u];
     __syncwarp();
-    warp_emit_units(su[warp], valid, out, keys, cap, err, hist ? shist : nullptr, hist ? hp.passes : 0u, hp.width);
+    warp_emit_units(su[warp], valid, out, keys, cap, err, shist, hp.passes, hp.width);
     __syncwarp();
   }
-  if (hist) {
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < hp.passes * 512; i += kScanBlock)
-      if (shist[i]) atomicAdd(hist + i, shist[i]);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < hp.passes * 512; i += kScanBlock)
+    if (shist[i]) atomicAdd(hist + i, shist[i]);
+}
+
+// The same from the rows that the count kept.  Finding a row's interval is
+// ~150 instructions, and the emission spent most of its time finding them
+// again.  Batch of 64 scenes (5.1M triangles, 41.7M keys): count 416 -> 497 us,
+// emission 850 -> 305 us; 4.2M-triangle soup: 154 -> 254 and 328 -> 120 us.
+template <class Maker>
+__global__ void __launch_bounds__(kScanBlock) k_emit_rows(Maker mk, uint32_t n, const uint32_t* __restrict__ offs,
+                                                         const uint2* __restrict__ rows,
+                                                         const uint2* __restrict__ gtab,
+                                                         uint64_t* __restrict__ keys, uint32_t cap, uint32_t* err,
+                                                         uint32_t* hist, SortPlan hp) {
+  __shared__ uint32_t shist[4 * 512];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < 4 * 512; i += kScanBlock) shist[i] = 0u;
+  __syncthreads();
+  const uint32_t groups = (n + 31u) / 32u;
+  for (uint32_t gi = blockIdx.x * kUnitWarps + warp; gi < groups; gi += gridDim.x * kUnitWarps) {
+    const uint2 G = gtab[gi];
+    if (G.x == kNoRows) continue;
+    const uint32_t i = gi * 32u + lane;
+    uint32_t id = 0, stride[2] = {0, 0};
+    if (i < n) mk.item(i, id, stride);
+    uint32_t out = offs[gi * 32u];
+    for (uint32_t k = 0; k < G.y; k += 32) {
+      uint2 row = make_uint2(0u, 0u);
+      if (k + lane < G.y) row = __ldcs(rows + G.x + k + lane);
+      const int ow = (int)((row.y >> 12) & 31u);
+      const uint32_t r = row.y >> 17;
+      const uint32_t rid = __shfl_sync(0xFFFFFFFFu, id, ow), s0 = __shfl_sync(0xFFFFFFFFu, stride[0], ow),
+                     s1 = __shfl_sync(0xFFFFFFFFu, stride[1], ow);
+      out += warp_emit_rows(row.x, row.y & 0xFFFu, r == 0u ? 1u : (r == 1u ? s0 : s1), rid, out, keys, cap, err, shist,
+                            hp.passes, hp.width);
+    }
   }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < hp.passes * 512; i += kScanBlock)
+    if (shist[i]) atomicAdd(hist + i, shist[i]);
 }
 
 // ---- precise (SAT) insertion --------------------------------------------------------
@@ -874,6 +923,12 @@ struct BatchMaker {
   const uint32_t* tri_off;
   const BatchScene* scenes;
   uint32_t ns;
+  SHN_D void item(uint32_t t, uint32_t& id, uint32_t stride[2]) const {
+    const Geom& g = scenes[find_segment(tri_off, ns, t)].g;
+    id = t;
+    stride[0] = (uint32_t)g.resf.x;
+    stride[1] = (uint32_t)(g.resf.x * g.resf.y);
+  }
   SHN_D bool operator()(uint32_t t, Unit& U) const {
     const uint32_t s = find_segment(tri_off, ns, t);
     V3 a, b, c;
@@ -888,18 +943,46 @@ int grid_for(uint64_t n, int block, int max_blocks) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(b, (uint64_t)max_blocks));
 }
 
+// Workspace of launch_counts for n items: look-back status, scan ticket and
+// group counter, reserved rows, and per group of 32 items its kept rows.
+size_t counts_bytes(uint64_t n) {
+  return ((n + kScanTile - 1) / kScanTile + 3) * 8 + ((n + 31) / 32) * sizeof(uint2);
+}
+
+RowStore row_store(void* ws, uint64_t n, uint2* rows, uint64_t cap) {
+  uint64_t* status = (uint64_t*)ws;
+  const size_t tiles = (n + kScanTile - 1) / kScanTile;
+  return RowStore{rows, std::min<uint64_t>(cap, kNoRows - 1u), (unsigned long long*)(status + tiles + 2),
+                  (uint2*)(status + tiles + 3)};
+}
+
 // Exact counts of n items into offs[0..n) then the in-place scan: offs[i] =
-// first output slot of item i, offs[n] = total.  ws: (tiles + 2) * 8 bytes
-// (look-back status, scan ticket, count group counter), zeroed here.
+// first output slot of item i, offs[n] = total.  ws: counts_bytes(n), cleared
+// here as far as needed.  rows (optional): room for `cap` rows, kept for
+// launch_emit.
 template <class Maker>
-void launch_counts(Maker mk, uint32_t n, uint32_t* offs, void* ws, uint32_t* err, cudaStream_t st) {
+void launch_counts(Maker mk, uint32_t n, uint32_t* offs, void* ws, uint2* rows, uint64_t cap, uint32_t* err,
+                   cudaStream_t st) {
   const size_t tiles = ((size_t)n + kScanTile - 1) / kScanTile;
   uint64_t* status = (uint64_t*)ws;
-  cudaMemsetAsync(status, 0, (tiles + 2) * 8, st);
+  cudaMemsetAsync(status, 0, (tiles + 3) * 8, st);
   uint32_t* ticket = (uint32_t*)(status + tiles + 1);
   const int blocks = grid_for((n + 31) / 32, kUnitWarps, 148 * 7);
-  k_count_groups<<<blocks, kScanBlock, 0, st>>>(mk, n, offs, ticket + 1);
+  k_count_groups<<<blocks, kScanBlock, 0, st>>>(mk, n, offs, ticket + 1, row_store(ws, n, rows, cap));
   k_scan_inplace<<<(unsigned)tiles, kScanBlock, 0, st>>>(offs, n, LookbackState{status, ticket, err});
+}
+
+// Emit grid: groups of 32 items, kUnitWarps groups per block step.
+int emit_blocks(uint64_t n) { return grid_for((n + 31) / 32, kUnitWarps, 148 * 8); }
+
+// The keys of the counted items.  rows: as given to launch_counts; some of the
+// groups' rows may not have been kept if `missing`.
+template <class Maker>
+void launch_emit(Maker mk, uint32_t n, const uint32_t* offs, void* ws, const uint2* rows, bool missing,
+                 uint64_t* keys, uint32_t cap, uint32_t* err, uint32_t* hist, SortPlan hp, cudaStream_t st) {
+  const uint2* gtab = rows ? row_store(ws, n, nullptr, 0).groups : nullptr;
+  if (rows) k_emit_rows<<<emit_blocks(n), kScanBlock, 0, st>>>(mk, n, offs, rows, gtab, keys, cap, err, hist, hp);
+  if (!rows || missing) k_emit_units<<<emit_blocks(n), kScanBlock, 0, st>>>(mk, n, offs, keys, cap, err, hist, hp, gtab);
 }
 
 // The counts and offsets of the precise insertion (as launch_counts).
@@ -979,6 +1062,19 @@ shn_status ensure_buf(shn_grid* g, DevBuf& b, size_t bytes, cudaStream_t st) {
   return ensure(g, &b.ptr, &b.bytes, bytes, st);
 }
 
+// Room for the rows of n items in key buffer `buf`, which the sort does not
+// need before the emission has read them: kRowsPerItem per item (the buffer
+// ends up about as large for the keys), or what the buffer has.  0 when the
+// budget or the device has no room for them: the emission then finds the rows
+// again.
+constexpr uint64_t kRowsPerItem = 6;
+
+uint64_t rows_room(shn_grid* g, int buf, uint64_t n, cudaStream_t st) {
+  const size_t want = std::min<uint64_t>(n * kRowsPerItem, 1ull << 30) * sizeof(uint2);
+  if (g->keys[buf].bytes < want && ensure_buf(g, g->keys[buf], want, st) != SHN_OK) return 0;
+  return g->keys[buf].bytes / sizeof(uint2);
+}
+
 LookbackState scan_state(shn_grid* g, uint64_t n, cudaStream_t st, shn_status* rc) {
   const size_t tiles = ((size_t)n + kScanTile - 1) / kScanTile;
   *rc = ensure_buf(g, g->scan, (tiles + 2) * 8, st);
@@ -989,9 +1085,6 @@ LookbackState scan_state(shn_grid* g, uint64_t n, cudaStream_t st, shn_status* r
 }
 
 int range_blocks(uint64_t n) { return grid_for(n, kRangeBlock * kRangeItems, 148 * 8); }
-
-// Emit grid: groups of 32 items, kUnitWarps groups per block step.
-int emit_blocks(uint64_t n) { return grid_for((n + 31) / 32, kUnitWarps, 148 * 8); }
 
 uint32_t scan_tiles(uint64_t n) { return (uint32_t)std::max<uint64_t>(1, (n + kScanTile - 1) / kScanTile); }
 
@@ -1103,18 +1196,26 @@ shn_status build_grid(shn_grid* g, const shn_scene* s, const shn_grid_params* p,
   if ((rc = ensure_buf(g, g->offs_tri, ((size_t)nt + 1) * 4, st))) return rc;
   uint32_t* offs = (uint32_t*)g->offs_tri.ptr;
   uint32_t P = 0;
+  uint64_t row_cap = 0, row_num = 0;  // room for kept rows in keys[1], rows found
   if (nt) {
-    if ((rc = ensure_buf(g, g->scan, (((size_t)nt + kScanTile - 1) / kScanTile + 2) * 8, st))) return rc;
+    if ((rc = ensure_buf(g, g->scan, counts_bytes(nt), st))) return rc;
+    if (!sat) row_cap = rows_room(g, 1, nt, st);
     if (sat) launch_counts_sat(tri, g->geom, nt, offs, g->scan.ptr, g->d_err, st);
-    else launch_counts(TopMaker{tri, g->geom}, nt, offs, g->scan.ptr, g->d_err, st);
-    const uint32_t* src[1] = {offs + nt};
-    if ((rc = read_words(g, src, 1, &P, st))) return rc;
+    else launch_counts(TopMaker{tri, g->geom}, nt, offs, g->scan.ptr, (uint2*)g->keys[1].ptr, row_cap, g->d_err, st);
+    const unsigned long long* next = row_store(g->scan.ptr, nt, nullptr, 0).next;
+    const uint32_t* src[3] = {offs + nt, (const uint32_t*)next, (const uint32_t*)next + 1};
+    uint32_t got[3] = {0, 0, 0};
+    if ((rc = read_words(g, src, sat ? 1 : 3, got, st))) return rc;
+    P = got[0];
+    row_num = got[1] | (uint64_t)got[2] << 32;
   }
   if (P >= (1u << 30)) return set_error(ctx, SHN_ERR_INVALID, "more than 2^30 cell references");
 
   // ---- emit + sort (uniform grid / top level) ----------------------------------
+  const size_t key_bytes = (size_t)std::max<uint32_t>(P, 1) * 8;
+  if (g->keys[1].bytes < key_bytes) row_cap = 0;  // the buffer that holds the rows is replaced
   for (int i = 0; i < 2; ++i)
-    if ((rc = ensure_buf(g, g->keys[i], (size_t)std::max<uint32_t>(P, 1) * 8, st))) return rc;
+    if ((rc = ensure_buf(g, g->keys[i], key_bytes, st))) return rc;
   if ((rc = ensure_buf(g, g->sortws, sort_workspace_bytes(P), st))) return rc;
   uint64_t* k0 = (uint64_t*)g->keys[0].ptr;
   uint64_t* k1 = (uint64_t*)g->keys[1].ptr;
@@ -1124,8 +1225,8 @@ shn_status build_grid(shn_grid* g, const shn_scene* s, const shn_grid_params* p,
     k_emit_sat<<<grid_for(nt, kScanBlock, 148 * 8), kScanBlock, 0, st>>>(tri, nt, g->geom, offs, k0, P, g->d_err,
                                                                         sort_hist_counts(g->sortws.ptr), top_plan);
   else if (nt)
-    k_emit_units<<<emit_blocks(nt), kScanBlock, 0, st>>>(TopMaker{tri, g->geom}, nt, offs, k0, P, g->d_err,
-                                                        sort_hist_counts(g->sortws.ptr), top_plan);
+    launch_emit(TopMaker{tri, g->geom}, nt, offs, g->scan.ptr, row_cap ? (const uint2*)k1 : nullptr, row_num > row_cap,
+                k0, P, g->d_err, sort_hist_counts(g->sortws.ptr), top_plan, st);
   uint64_t* sortedTop = onesweep_sort(k0, k1, P, 32, top_plan, g->sortws.ptr, g->d_err, st, true);
   const int topBuf = sortedTop == k0 ? 0 : 1;
 
@@ -1170,20 +1271,26 @@ shn_status build_grid(shn_grid* g, const shn_scene* s, const shn_grid_params* p,
   }
   if ((rc = ensure_buf(g, g->offs_pair, ((size_t)P + 1) * 4, st))) return rc;
   uint32_t* pairOffs = (uint32_t*)g->offs_pair.ptr;
+  const int bA = (topBuf + 1) % 3, bB = (topBuf + 2) % 3;
+  row_cap = row_num = 0;
   if (P) {
-    if ((rc = ensure_buf(g, g->scan, (((size_t)P + kScanTile - 1) / kScanTile + 2) * 8, st))) return rc;
-    launch_counts(LeafMaker{tri, sortedTop, g->cells, g->geom}, P, pairOffs, g->scan.ptr, g->d_err, st);
+    if ((rc = ensure_buf(g, g->scan, counts_bytes(P), st))) return rc;
+    row_cap = rows_room(g, bB, P, st);
+    launch_counts(LeafMaker{tri, sortedTop, g->cells, g->geom}, P, pairOffs, g->scan.ptr, (uint2*)g->keys[bB].ptr,
+                  row_cap, g->d_err, st);
   } else {
     cudaMemsetAsync(pairOffs, 0, 4, st);
   }
-  uint32_t sizes[2];
+  uint32_t sizes[4] = {0, 0, 0, 0};
   {
-    const uint32_t* src[2] = {d_L, pairOffs + P};
-    if ((rc = read_words(g, src, 2, sizes, st))) return rc;
+    const unsigned long long* next = row_store(g->scan.ptr, P, nullptr, 0).next;
+    const uint32_t* src[4] = {d_L, pairOffs + P, (const uint32_t*)next, (const uint32_t*)next + 1};
+    if ((rc = read_words(g, src, P ? 4 : 2, sizes, st))) return rc;
+    row_num = sizes[2] | (uint64_t)sizes[3] << 32;
   }
   const uint32_t Lc = sizes[0], R = sizes[1];
   if (R >= (1u << 30)) return set_error(ctx, SHN_ERR_INVALID, "more than 2^30 leaf references");
-  const int bA = (topBuf + 1) % 3, bB = (topBuf + 2) % 3;
+  if (g->keys[bB].bytes < (size_t)std::max<uint32_t>(R, 1) * 8) row_cap = 0;
   if ((rc = ensure_buf(g, g->keys[bA], (size_t)std::max<uint32_t>(R, 1) * 8, st))) return rc;
   if ((rc = ensure_buf(g, g->keys[bB], (size_t)std::max<uint32_t>(R, 1) * 8, st))) return rc;
   if ((rc = ensure_buf(g, g->sortws, sort_workspace_bytes(R), st))) return rc;
@@ -1192,9 +1299,9 @@ shn_status build_grid(shn_grid* g, const shn_scene* s, const shn_grid_params* p,
   const SortPlan leaf_plan = sort_plan(key_bits_for(Lc ? Lc - 1 : 0));
   sort_prepare(g->sortws.ptr, st);
   if (P)
-    k_emit_units<<<emit_blocks(P), kScanBlock, 0, st>>>(LeafMaker{tri, sortedTop, g->cells, g->geom}, P,
-                                                       pairOffs, lk0, R, g->d_err,
-                                                       sort_hist_counts(g->sortws.ptr), leaf_plan);
+    launch_emit(LeafMaker{tri, sortedTop, g->cells, g->geom}, P, pairOffs, g->scan.ptr,
+                row_cap ? (const uint2*)lk1 : nullptr, row_num > row_cap, lk0, R, g->d_err,
+                sort_hist_counts(g->sortws.ptr), leaf_plan, st);
   uint64_t* sortedLeaf = onesweep_sort(lk0, lk1, R, 32, leaf_plan, g->sortws.ptr, g->d_err, st, true);
   if ((rc = ensure(g, (void**)&g->leaves, &g->cap_leaves, (size_t)std::max<uint32_t>(Lc, 1) * 8, st))) return rc;
   if ((rc = ensure(g, (void**)&g->indices, &g->cap_refs, (size_t)std::max<uint32_t>(R, 1) * 4, st))) return rc;
@@ -1247,25 +1354,30 @@ void launch_batch_bounds(const float4* tri, const uint32_t* tri_off, uint32_t ns
   k_batch_bounds_decode<<<(6 * ns + 255) / 256, 256, 0, st>>>((uint32_t*)d_out6ns, 6 * ns);
 }
 
-size_t batch_scan_bytes(uint32_t T) { return (((size_t)T + kScanTile - 1) / kScanTile + 2) * 8; }
+size_t batch_scan_bytes(uint32_t T) { return counts_bytes(T); }
+
+const uint64_t* batch_row_count(void* scan_ws, uint32_t T) {
+  return (const uint64_t*)row_store(scan_ws, T, nullptr, 0).next;
+}
 
 void launch_batch_count(const float4* tri, uint32_t T, const uint32_t* tri_off, const BatchScene* scenes,
-                        uint32_t ns, void* scan_ws, uint32_t* err, uint32_t* offs, cudaStream_t st) {
+                        uint32_t ns, void* scan_ws, void* rows, uint64_t row_cap, uint32_t* err, uint32_t* offs,
+                        cudaStream_t st) {
   if (!T) {
     cudaMemsetAsync(offs, 0, 4, st);
     return;
   }
   const TriArr ts{tri};
-  launch_counts(BatchMaker{ts, tri_off, scenes, ns}, T, offs, scan_ws, err, st);
+  launch_counts(BatchMaker{ts, tri_off, scenes, ns}, T, offs, scan_ws, (uint2*)rows, row_cap, err, st);
 }
 
 void launch_batch_emit(const float4* tri, uint32_t T, const uint32_t* tri_off, const BatchScene* scenes,
-                       uint32_t ns, const uint32_t* offs, uint64_t* keys, uint32_t capacity,
-                       uint32_t* err, uint32_t* hist, SortPlan hplan, cudaStream_t st) {
+                       uint32_t ns, const uint32_t* offs, void* scan_ws, const void* rows, uint64_t* keys,
+                       uint32_t capacity, uint32_t* err, uint32_t* hist, SortPlan hplan, cudaStream_t st) {
   const TriArr ts{tri};
   if (T)
-    k_emit_units<<<emit_blocks(T), kScanBlock, 0, st>>>(BatchMaker{ts, tri_off, scenes, ns}, T, offs, keys,
-                                                       capacity, err, hist, hplan);
+    launch_emit(BatchMaker{ts, tri_off, scenes, ns}, T, offs, scan_ws, (const uint2*)rows, false, keys, capacity, err,
+                hist, hplan, st);
 }
 
 void launch_cell_ranges(const uint64_t* keys, uint32_t n, uint64_t C, uint2* ranges, uint32_t* indices,

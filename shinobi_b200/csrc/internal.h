@@ -175,10 +175,14 @@ void launch_batch_bounds(const float4* tri, const uint32_t* tri_off, uint32_t ns
                          float* d_out6ns, cudaStream_t st);
 size_t batch_scan_bytes(uint32_t T);
 void launch_batch_count(const float4* tri, uint32_t T, const uint32_t* tri_off, const BatchScene* scenes,
-                        uint32_t ns, void* scan_ws, uint32_t* err, uint32_t* offs, cudaStream_t st);
+                        uint32_t ns, void* scan_ws, void* rows, uint64_t row_cap, uint32_t* err, uint32_t* offs,
+                        cudaStream_t st);
+// rows found by the last count (device word); rows/row_cap: 8-byte slots in
+// which they are kept for the emission (all of them must fit), or null
+const uint64_t* batch_row_count(void* scan_ws, uint32_t T);
 void launch_batch_emit(const float4* tri, uint32_t T, const uint32_t* tri_off, const BatchScene* scenes,
-                       uint32_t ns, const uint32_t* offs, uint64_t* keys, uint32_t capacity,
-                       uint32_t* err, uint32_t* hist, SortPlan hplan, cudaStream_t st);
+                       uint32_t ns, const uint32_t* offs, void* scan_ws, const void* rows, uint64_t* keys,
+                       uint32_t capacity, uint32_t* err, uint32_t* hist, SortPlan hplan, cudaStream_t st);
 // Ranges of all C cells (empty ones (0, 0)) and indices[], written by tiles
 // of cells: needs no cleared cell array.
 // (key's triangle + id0)

@@ -58,7 +58,7 @@ struct Unit {
   float R;             // min_k (s_k/2 + eps)/|n_k|  (estimate only)
   float inv_nr;        // 1/n_r                      (estimate only)
   float inv_sr;        // 1/s_r                      (estimate only)
-  uint32_t pad;
+  float inv_su;        // 1/span[u], u the first axis across the row
 };
 
 SHN_HD void unit_axes(int r, int& u, int& v) {
@@ -84,7 +84,9 @@ SHN_HD void unit_finish(Unit& U, bool plane) {
     U.inv_nr = 0.f;
     U.inv_sr = 0.f;
   }
-  U.pad = 0u;
+  int u, v;
+  unit_axes(r, u, v);
+  U.inv_su = 1.0f / (float)U.span[u];
 }
 
 SHN_HD uint32_t unit_rows(const Unit& U) {
@@ -100,6 +102,16 @@ SHN_HD float acc_centre(const Unit& U, int k, uint32_t i) {
   float c = (((float)U.lo[k] * s + U.o[k]) + s * 0.5f) - s;
   for (uint32_t q = U.lo[k]; q <= i; ++q) c += s;
   return c;
+}
+
+// The indices of row j across the row axis.  (j + 1/2) / span in floats: below
+// 2^21 its error, 2^-23 of the quotient, stays under the 1/2 / span that keep
+// it from the next integer.
+SHN_HD void unit_cross(const Unit& U, int u, int v, uint32_t j, uint32_t& iu, uint32_t& iv) {
+  const uint32_t su = U.span[u];
+  const uint32_t q = j < (1u << 21) ? (uint32_t)(((float)j + 0.5f) * U.inv_su) : j / su;
+  iu = U.lo[u] + (j - q * su);
+  iv = U.lo[v] + q;
 }
 
 // (c_k(i) - a_k) * n_k
@@ -132,8 +144,8 @@ SHN_HD void row_interval(const Unit& U, uint32_t j, uint32_t& f, uint32_t& e) {
   const int r = (int)(U.meta & 3u);
   int u, v;
   unit_axes(r, u, v);
-  const uint32_t su = U.span[u];
-  const uint32_t iu = U.lo[u] + j % su, iv = U.lo[v] + j / su;
+  uint32_t iu, iv;
+  unit_cross(U, u, v, j, iu, iv);
   const float tu = unit_term(U, u, iu), tv = unit_term(U, v, iv);
   const uint32_t lo = U.lo[r], hi1 = U.lo[r] + U.span[r];  // [lo, hi1)
   const float s = U.s[r];
@@ -215,52 +227,114 @@ SHN_D uint32_t warp_incl_sum(uint32_t v) {
   return v;
 }
 
+// First cell, number and axis of the passing cells of row j of unit W.
+SHN_D void unit_row(const Unit& W, uint32_t j, uint32_t& c0, uint32_t& len, int& r) {
+  r = (int)(W.meta & 3u);
+  int u, v;
+  unit_axes(r, u, v);
+  uint32_t f, e;
+  if (W.meta & 4u) {
+    row_interval(W, j, f, e);
+  } else {
+    f = W.lo[r];
+    e = W.lo[r] + W.span[r];
+  }
+  len = e - f;
+  uint32_t iu, iv;
+  unit_cross(W, u, v, j, iu, iv);
+  uint32_t x, y, z;
+  if (r == 0) { x = f; y = iu; z = iv; }
+  else if (r == 1) { x = iu; y = f; z = iv; }
+  else { x = iu; y = iv; z = f; }
+  c0 = W.base + x + y * W.stride[0] + z * W.stride[1];
+}
+
+// The rows found while counting, kept for the emission: per group of 32 items
+// a run of (first cell, length | item in the group << 12 | axis << 17), the
+// rows with passing cells in order.  A group whose rows (empty ones included)
+// do not fit is marked and found again by the emission.
+struct RowStore {
+  uint2* rows;               // null: nothing is kept
+  uint64_t cap;
+  unsigned long long* next;  // rows reserved so far (counted without a store, too)
+  uint2* groups;             // per group: first row (kNoRows: not kept), number of rows
+};
+constexpr uint32_t kNoRows = 0xFFFFFFFFu;
+
 // Candidate count of every lane's unit (after the plane test).  su: the
 // warp's 32 unit slots in shared memory, slot `lane` filled by this lane when
-// `valid`; acc: 32 words of shared memory.
-SHN_D uint32_t warp_count_units(Unit* su, uint32_t* acc, bool valid) {
+// `valid`; acc: 32 words of shared memory; group: number of the 32 items.
+SHN_D uint32_t warp_count_units(Unit* su, uint32_t* acc, bool valid, const RowStore& S, uint32_t group) {
   const int lane = threadIdx.x & 31;
-  const bool plane = valid && (su[lane].meta & 4u);
-  const uint32_t direct = (valid && !plane) ? unit_cells(su[lane]) : 0u;
-  const uint32_t rows = plane ? unit_rows(su[lane]) : 0u;
+  const uint32_t rows = valid ? unit_rows(su[lane]) : 0u;
   acc[lane] = 0u;
   const uint32_t incl = warp_incl_sum(rows);
   const uint32_t tot = __shfl_sync(kWarpFull, incl, 31);
   const uint32_t pre = incl - rows;
+  uint32_t start = kNoRows;
+  if (lane == 0 && tot) {
+    const unsigned long long at = atomicAdd(S.next, (unsigned long long)tot);
+    if (S.rows && at + tot <= S.cap) start = (uint32_t)at;
+  }
+  start = __shfl_sync(kWarpFull, start, 0);
+  uint32_t kept = 0;
   __syncwarp();
   for (uint32_t j0 = 0; j0 < tot; j0 += 32) {
     const uint32_t j = j0 + lane;
     const int ow = warp_search(pre, j);
     const uint32_t opre = __shfl_sync(kWarpFull, pre, ow);
-    uint32_t len = 0;
-    if (j < tot) {
-      uint32_t f, e;
-      row_interval(su[ow], j - opre, f, e);
-      len = e - f;
+    uint32_t len = 0, c0 = 0;
+    int r = 0;
+    if (j < tot) unit_row(su[ow], j - opre, c0, len, r);
+    if (start != kNoRows) {
+      const uint32_t m = __ballot_sync(kWarpFull, len != 0u);
+      if (len) S.rows[start + kept + __popc(m & ((1u << lane) - 1u))] = make_uint2(c0, len | (uint32_t)ow << 12 | (uint32_t)r << 17);
+      kept += __popc(m);
     }
-    // segmented sum over lanes with the same owner (owners are non-decreasing)
-    uint32_t sum = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(kWarpFull, sum, o);
-      const int w = __shfl_up_sync(kWarpFull, ow, o);
-      if (lane >= o && w == ow) sum += y;
-    }
-    const int nxt = __shfl_down_sync(kWarpFull, ow, 1);
-    if ((lane == 31 || nxt != ow) && sum) acc[ow] += sum;  // one writer per owner
-    __syncwarp();
+    if (len) atomicAdd(acc + ow, len);
   }
-  return direct + acc[lane];
+  __syncwarp();
+  if (lane == 0 && S.groups) S.groups[group] = make_uint2(tot ? start : 0u, kept);
+  return acc[lane];
+}
+
+// Keys of 32 rows at a time: row `lane` has len cells from c0 on, st apart, of
+// item id.  Writes them to keys[out ...] in order and returns their number.
+// Stores beyond `cap` are dropped and flagged with kErrCapacity.  When shist
+// is non-null, the hwidth-bit digits (cell >> hwidth*p) of every key, p <
+// hpasses, are counted into shist[p * 512 + digit] (shared memory).
+SHN_D uint32_t warp_emit_rows(uint32_t c0, uint32_t len, uint32_t st, uint32_t id, uint32_t out,
+                              uint64_t* __restrict__ keys, uint32_t cap, uint32_t* err, uint32_t* shist,
+                              uint32_t hpasses, uint32_t hwidth) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t pincl = warp_incl_sum(len);
+  const uint32_t L = __shfl_sync(kWarpFull, pincl, 31);
+  const uint32_t pos = pincl - len;
+  // the cells are below 2^bits of the sort plan: the last pass's digit needs
+  // no narrower mask
+  const uint32_t hmask = (1u << hwidth) - 1u;
+  for (uint32_t q0 = 0; q0 < L; q0 += 32) {
+    const uint32_t q = q0 + lane;
+    const int src = warp_search(pos, q);
+    const uint32_t sc = __shfl_sync(kWarpFull, c0, src);
+    const uint32_t ss = __shfl_sync(kWarpFull, st, src);
+    const uint32_t sid = __shfl_sync(kWarpFull, id, src);
+    const uint32_t sp = __shfl_sync(kWarpFull, pos, src);
+    if (q < L) {
+      const uint32_t o = out + q;
+      const uint32_t cell = sc + (q - sp) * ss;
+      if (o < cap) __stcs(keys + o, ((uint64_t)cell << 32) | sid);
+      else atomicOr(err, kErrCapacity);
+      for (uint32_t p = 0; p < hpasses; ++p) atomicAdd(shist + p * 512 + ((cell >> (hwidth * p)) & hmask), 1u);
+    }
+  }
+  return L;
 }
 
 // Writes the keys (cell << 32 | id) of the 32 lanes' units (slots filled as
 // for warp_count_units), unit after unit and row after row, to keys[out ...].
-// Stores beyond `cap` are dropped and flagged with kErrCapacity.  When shist
-// is non-null, the hwidth-bit digits (cell >> hwidth*p) of every key, p <
-// hpasses, are counted into shist[p * 512 + digit] (shared memory).
 SHN_D void warp_emit_units(Unit* su, bool valid, uint32_t out, uint64_t* __restrict__ keys, uint32_t cap,
-                           uint32_t* err, uint32_t* shist = nullptr, uint32_t hpasses = 0,
-                           uint32_t hwidth = 8) {
+                           uint32_t* err, uint32_t* shist, uint32_t hpasses, uint32_t hwidth) {
   const int lane = threadIdx.x & 31;
   const uint32_t rows = valid ? unit_rows(su[lane]) : 0u;
   const uint32_t incl = warp_incl_sum(rows);
@@ -274,49 +348,12 @@ SHN_D void warp_emit_units(Unit* su, bool valid, uint32_t out, uint64_t* __restr
     uint32_t len = 0, c0 = 0, st = 0, id = 0;
     if (j < tot) {
       const Unit& W = su[ow];
-      const uint32_t jr = j - opre;
-      const int r = (int)(W.meta & 3u);
-      int u, v;
-      unit_axes(r, u, v);
-      uint32_t f, e;
-      if (W.meta & 4u) {
-        row_interval(W, jr, f, e);
-      } else {
-        f = W.lo[r];
-        e = W.lo[r] + W.span[r];
-      }
-      len = e - f;
-      const uint32_t iu = W.lo[u] + jr % W.span[u], iv = W.lo[v] + jr / W.span[u];
-      uint32_t x, y, z;
-      if (r == 0) { x = f; y = iu; z = iv; }
-      else if (r == 1) { x = iu; y = f; z = iv; }
-      else { x = iu; y = iv; z = f; }
-      c0 = W.base + x + y * W.stride[0] + z * W.stride[1];
+      int r;
+      unit_row(W, j - opre, c0, len, r);
       st = r == 0 ? 1u : W.stride[r - 1];
       id = W.id;
     }
-    const uint32_t pincl = warp_incl_sum(len);
-    const uint32_t L = __shfl_sync(kWarpFull, pincl, 31);
-    const uint32_t pos = pincl - len;
-    for (uint32_t q0 = 0; q0 < L; q0 += 32) {
-      const uint32_t q = q0 + lane;
-      const int src = warp_search(pos, q);
-      const uint32_t sc = __shfl_sync(kWarpFull, c0, src);
-      const uint32_t ss = __shfl_sync(kWarpFull, st, src);
-      const uint32_t sid = __shfl_sync(kWarpFull, id, src);
-      const uint32_t sp = __shfl_sync(kWarpFull, pos, src);
-      if (q < L) {
-        const uint32_t o = out + q;
-        const uint32_t cell = sc + (q - sp) * ss;
-        if (o < cap) __stcs(keys + o, ((uint64_t)cell << 32) | sid);
-        else atomicOr(err, kErrCapacity);
-        // the cells are below 2^bits of the sort plan: the last pass's digit
-        // needs no narrower mask
-        const uint32_t hmask = (1u << hwidth) - 1u;
-        for (uint32_t p = 0; p < hpasses; ++p) atomicAdd(shist + p * 512 + ((cell >> (hwidth * p)) & hmask), 1u);
-      }
-    }
-    out += L;
+    out += warp_emit_rows(c0, len, st, id, out, keys, cap, err, shist, hpasses, hwidth);
     __syncwarp();
   }
 }

@@ -6,7 +6,8 @@
 //  * the digit counts of every pass come from one histogram kernel over the
 //    keys, or from the producer of the keys while it writes them (the grid
 //    build's key emission does this; see sort_hist_counts);
-//  * each pass is ONE kernel over 6144-key tiles (two per SM): a tile is staged into
+//  * each pass is ONE kernel over 6144-key tiles (two per SM; smaller ones for
+//    few keys): a tile is staged into
 //    shared memory with a bulk asynchronous copy (cp.async.bulk +
 //    mbarrier), each warp's digit counts are taken with order-free shared
 //    atomics, the tile's counts are published at once and combined across
@@ -298,12 +299,22 @@ __global__ void __launch_bounds__(kSortBlock, MINB) k_onesweep(const uint64_t* _
 
 }  // namespace
 
-size_t sort_workspace_bytes(uint32_t n) {
-  const size_t tiles = ((size_t)n + kMinTile - 1) / kMinTile;
-  return (4 * kMaxBins + 8) * sizeof(uint32_t) + tiles * kMaxBins * sizeof(uint32_t);
+// Keys per thread of a sort of n keys.  A pass over few keys is one wave of
+// tiles and takes as long as a tile, so up to one wave (two tiles per SM) the
+// tiles get smaller: 4 keys per thread (2048-key tiles) up to 296 tiles of
+// them, then 8 likewise.  Frames of the 262,144-triangle cluster 2.56 -> 2.49 ms
+// per two rebuilds and renders, the 65,536-triangle frame 304 -> 298 us, the
+// 1M-triangle frame 4.98 -> 4.95 ms.
+constexpr uint32_t kWave = 2 * 148;
+static int sort_items(uint32_t n) {
+  return n <= kWave * kSortBlock * 4 ? 4 : (n <= kWave * kSortBlock * 8 ? 8 : kPassItems);
 }
 
-uint32_t sort_tiles(uint32_t n) { return (uint32_t)(((size_t)n + kMinTile - 1) / kMinTile); }
+size_t sort_workspace_bytes(uint32_t n) {
+  const size_t tile = std::min(kMinTile, kSortBlock * sort_items(n));
+  const size_t tiles = ((size_t)n + tile - 1) / tile;
+  return (4 * kMaxBins + 8) * sizeof(uint32_t) + tiles * kMaxBins * sizeof(uint32_t);
+}
 
 uint32_t* sort_hist_counts(void* ws) { return (uint32_t*)ws; }
 
@@ -379,12 +390,14 @@ uint64_t* onesweep_sort(uint64_t* buf0, uint64_t* buf1, uint32_t n, uint32_t lo_
     const uint32_t w = std::min(plan.width, plan.bits - plan.width * p);
     const uint32_t mask = (1u << w) - 1u;
     // 4096-key tiles (8 per thread) are the autotuner's alternative tile shape
-    const bool t4k = tile_keys == 4096u;
+    const int items = tile_keys == 4096u ? 8 : (tile_keys ? kPassItems : sort_items(n));
     if (plan.width == 9) {
-      if (t4k) launch_pass<8, 2, 9>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
+      if (items == 4) launch_pass<4, 2, 9>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
+      else if (items == 8) launch_pass<8, 2, 9>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
       else launch_pass<kPassItems, 2, 9>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
     } else {
-      if (t4k) launch_pass<8, 2, 8>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
+      if (items == 4) launch_pass<4, 2, 8>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
+      else if (items == 8) launch_pass<8, 2, 8>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
       else launch_pass<kPassItems, 2, 8>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
     }
     std::swap(src, dst);

@@ -302,6 +302,17 @@ shn_status shn_trace_closest(const shn_grid* g, const shn_rays* rays, uint32_t n
 shn_status shn_trace_any(const shn_grid* g, const shn_rays* rays, uint32_t n, uint8_t* d_occluded,
                          void* stream);
 
+/* The same for rays whose coordinates are not contiguous: coordinate c of ray
+ * i is read at c[i * stride], in floats (an (n, 3) array has stride 3 and
+ * pointers to its columns; stride 0 repeats one value). */
+typedef struct shn_ray_strides {
+  int64_t org, dir, tmax;
+} shn_ray_strides;
+shn_status shn_trace_closest_strided(const shn_grid* g, const shn_rays* rays, const shn_ray_strides* strides,
+                                     uint32_t n, shn_hits* hits, void* stream);
+shn_status shn_trace_any_strided(const shn_grid* g, const shn_rays* rays, const shn_ray_strides* strides, uint32_t n,
+                                 uint8_t* d_occluded, void* stream);
+
 typedef struct shn_camera {
   float eye[3], forward[3], up[3];
   float fov_deg;            /* vertical opening angle */

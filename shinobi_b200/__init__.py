@@ -334,6 +334,20 @@ class Grid:
                 "res": np.array(inf.res[:], np.int32), "bounds": np.array(inf.bounds[:], np.float32)}
 
     @staticmethod
+    def _strided(org, dirs, tmax):
+        """Rays read in place: float32 device arrays (n, 3), (n, 3) and (n,) of any strides; None for others."""
+        torch = _torch()
+        if (org.ndim != 2 or dirs.ndim != 2 or org.shape[1] < 3 or dirs.shape[1] < 3 or dirs.shape[0] < org.shape[0]
+                or (tmax is not None and (tmax.ndim != 1 or tmax.shape[0] < org.shape[0]))):
+            return None
+        if any(x is not None and (x.dtype != torch.float32 or not x.is_cuda) for x in (org, dirs, tmax)):
+            return None
+        o, d, so, sd = org.data_ptr(), dirs.data_ptr(), org.stride(), dirs.stride()
+        r = _abi.Rays(*[o + 4 * k * so[1] for k in range(3)], *[d + 4 * k * sd[1] for k in range(3)],
+                      tmax.data_ptr() if tmax is not None else None)
+        return r, _abi.RayStrides(so[0], sd[0], tmax.stride(0) if tmax is not None else 0)
+
+    @staticmethod
     def _rays(org, dirs, tmax):
         cols = [org[:, k].contiguous() for k in range(3)] + [dirs[:, k].contiguous() for k in range(3)]
         r = _abi.Rays(*[_ptr(c) for c in cols], _ptr(tmax.contiguous()) if tmax is not None else None)
@@ -342,8 +356,13 @@ class Grid:
     def trace_closest(self, org, dirs, tmax=None, out: HitBuffers | None = None, stream=None) -> HitBuffers:
         n = org.shape[0]
         out = out or alloc_hits(n, org.device)
-        r, keep = self._rays(org, dirs, tmax)
         h = out.struct()
+        s = self._strided(org, dirs, tmax)
+        if s is not None:
+            self.ctx.check(self.ctx.lib.shn_trace_closest_strided(
+                self.handle, C.byref(s[0]), C.byref(s[1]), n, C.byref(h), _stream(stream)), "shn_trace_closest_strided")
+            return out
+        r, keep = self._rays(org, dirs, tmax)
         self.ctx.check(self.ctx.lib.shn_trace_closest(self.handle, C.byref(r), n, C.byref(h),
                                                       _stream(stream)), "shn_trace_closest")
         return out
@@ -352,6 +371,11 @@ class Grid:
         torch = _torch()
         n = org.shape[0]
         out = out if out is not None else torch.empty(n, dtype=torch.uint8, device=org.device)
+        s = self._strided(org, dirs, tmax)
+        if s is not None:
+            self.ctx.check(self.ctx.lib.shn_trace_any_strided(
+                self.handle, C.byref(s[0]), C.byref(s[1]), n, _ptr(out), _stream(stream)), "shn_trace_any_strided")
+            return out
         r, keep = self._rays(org, dirs, tmax)
         self.ctx.check(self.ctx.lib.shn_trace_any(self.handle, C.byref(r), n, _ptr(out),
                                                   _stream(stream)), "shn_trace_any")

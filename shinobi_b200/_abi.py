@@ -44,6 +44,10 @@ class Rays(C.Structure):
     _fields_ = [("ox", vp), ("oy", vp), ("oz", vp), ("dx", vp), ("dy", vp), ("dz", vp), ("tmax", vp)]
 
 
+class RayStrides(C.Structure):
+    _fields_ = [("org", C.c_int64), ("dir", C.c_int64), ("tmax", C.c_int64)]
+
+
 class Hits(C.Structure):
     _fields_ = [("tri", vp), ("t", vp), ("u", vp), ("v", vp)]
 
@@ -140,6 +144,8 @@ SIGNATURES = {
     "shn_grid_destroy": ([vp], None),
     "shn_trace_closest": ([vp, C.POINTER(Rays), u32, C.POINTER(Hits), vp], i32),
     "shn_trace_any": ([vp, C.POINTER(Rays), u32, vp, vp], i32),
+    "shn_trace_closest_strided": ([vp, C.POINTER(Rays), C.POINTER(RayStrides), u32, C.POINTER(Hits), vp], i32),
+    "shn_trace_any_strided": ([vp, C.POINTER(Rays), C.POINTER(RayStrides), u32, vp, vp], i32),
     "shn_trace_primary": ([vp, C.POINTER(Camera), u32, C.POINTER(Hits), vp], i32),
     "shn_trace_ao": ([vp, C.POINTER(Camera), C.POINTER(Hits), u32, f32, f32, u32, vp, vp, vp], i32),
     "shn_grid_set_stats": ([vp, vp], i32),

@@ -8,10 +8,6 @@ namespace shn {
 
 namespace {
 
-struct RaysView {
-  const float *ox, *oy, *oz, *dx, *dy, *dz, *tmax;
-};
-
 template <bool ANY>
 __global__ void __launch_bounds__(kCoopBlock, kFlatBlocks) k_flat_rays(const __grid_constant__ GridView G, RaysView R, uint32_t n, uint32_t* counter,
                                                            uint32_t* otri, float* ot, float* ou, float* ov,
@@ -20,9 +16,7 @@ __global__ void __launch_bounds__(kCoopBlock, kFlatBlocks) k_flat_rays(const __g
   flat_trace<ANY>(
       sm, FlatGrid{&G}, n, ou || ov, counter,
       [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) {
-        o = mk(__ldg(R.ox + i), __ldg(R.oy + i), __ldg(R.oz + i));
-        d = mk(__ldg(R.dx + i), __ldg(R.dy + i), __ldg(R.dz + i));
-        tmax = R.tmax ? __ldg(R.tmax + i) : FLT_MAX;
+        R.ray(i, o, d, tmax);
       },
       [&](uint32_t i, const Hit& h, uint32_t) {
         if (ANY) {
@@ -80,20 +74,18 @@ int flat_blocks(K kernel, int num_sms, uint64_t n) {
   return (int)std::min<uint64_t>((uint64_t)per_sm * num_sms, need);
 }
 
-RaysView view(const shn_rays& r) { return RaysView{r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.tmax}; }
-
 }  // namespace
 
-void launch_flat_closest(const GridView& G, const shn_rays& rays, uint32_t n, uint32_t* counter, const shn_hits& hits,
+void launch_flat_closest(const GridView& G, const RaysView& rays, uint32_t n, uint32_t* counter, const shn_hits& hits,
                          int num_sms, cudaStream_t st) {
   k_flat_rays<false><<<flat_blocks(k_flat_rays<false>, num_sms, n), kCoopBlock, 0, st>>>(
-      G, view(rays), n, counter, hits.tri, hits.t, hits.u, hits.v, nullptr);
+      G, rays, n, counter, hits.tri, hits.t, hits.u, hits.v, nullptr);
 }
 
-void launch_flat_any(const GridView& G, const shn_rays& rays, uint32_t n, uint32_t* counter, uint8_t* occ, int num_sms,
+void launch_flat_any(const GridView& G, const RaysView& rays, uint32_t n, uint32_t* counter, uint8_t* occ, int num_sms,
                      cudaStream_t st) {
   k_flat_rays<true><<<flat_blocks(k_flat_rays<true>, num_sms, n), kCoopBlock, 0, st>>>(
-      G, view(rays), n, counter, nullptr, nullptr, nullptr, nullptr, occ);
+      G, rays, n, counter, nullptr, nullptr, nullptr, nullptr, occ);
 }
 
 void launch_flat_camera(const GridView& G, const CamView& cam, uint32_t image_id, uint32_t n, uint32_t* counter,

@@ -191,13 +191,14 @@ void launch_cell_ranges(const uint64_t* keys, uint32_t n, uint64_t C, uint2* ran
 // trace.cu
 struct CamView;
 struct GridView;
+struct RaysView;
 CamView make_camera(const shn_camera* c);
 GridView view_of(const shn_grid* g);
 
 // flat.cu: uniform grids; counter is a zeroed device word
-void launch_flat_closest(const GridView& G, const shn_rays& rays, uint32_t n, uint32_t* counter, const shn_hits& hits,
+void launch_flat_closest(const GridView& G, const RaysView& rays, uint32_t n, uint32_t* counter, const shn_hits& hits,
                          int num_sms, cudaStream_t st);
-void launch_flat_any(const GridView& G, const shn_rays& rays, uint32_t n, uint32_t* counter, uint8_t* occ, int num_sms,
+void launch_flat_any(const GridView& G, const RaysView& rays, uint32_t n, uint32_t* counter, uint8_t* occ, int num_sms,
                      cudaStream_t st);
 struct AoRays;
 struct DiRays;

@@ -16,10 +16,6 @@ namespace {
 
 constexpr int kTraceBlock = 128;
 
-struct RaysView {
-  const float *ox, *oy, *oz, *dx, *dy, *dz, *tmax;
-};
-
 // Work counters of the stats variants: {cell visits, triangle tests}, warp-aggregated.
 template <bool STATS>
 SHN_D void add_stats(unsigned long long* stats, const Hit& h, bool valid) {
@@ -52,9 +48,7 @@ __global__ void __launch_bounds__(kTraceBlock, 8) k_trace_rays(GridView G, RaysV
   warp_trace<KIND, ANY>(
       G, n, counter,
       [&](uint32_t i, V3& o, V3& d, float& tmax) {
-        o = mk(R.ox[i], R.oy[i], R.oz[i]);
-        d = mk(R.dx[i], R.dy[i], R.dz[i]);
-        tmax = R.tmax ? R.tmax[i] : FLT_MAX;
+        R.ray(i, o, d, tmax);
       },
       [&](uint32_t i, const Hit& h, uint32_t steps, uint32_t tests) {
         if (ANY) {
@@ -247,6 +241,10 @@ void trace_from_hits(const shn_grid* g, const GridView& G, const Rays& R, const 
 #undef SHN_LAUNCH_HITS
 }
 
+RaysView view_rays(const shn_rays& r, const shn_ray_strides* s) {
+  return RaysView{r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.tmax, s ? s->org : 1, s ? s->dir : 1, s ? s->tmax : 1};
+}
+
 shn_status check_launch(shn_ctx* ctx, const char* what) {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SHN_OK : cuda_status(ctx, e, what);
@@ -308,6 +306,11 @@ shn_status shn_grid_set_stats(shn_grid* g, uint64_t* d_counters) {
 
 shn_status shn_trace_closest(const shn_grid* g, const shn_rays* rays, uint32_t n, shn_hits* hits,
                              void* stream) {
+  return shn_trace_closest_strided(g, rays, nullptr, n, hits, stream);
+}
+
+shn_status shn_trace_closest_strided(const shn_grid* g, const shn_rays* rays, const shn_ray_strides* strides,
+                                     uint32_t n, shn_hits* hits, void* stream) {
   if (!g || !rays || !hits) return SHN_ERR_INVALID;
   if (!g->built) return set_error(g->ctx, SHN_ERR_NOT_BUILT, "grid not built");
   grid_fence(g, (cudaStream_t)stream);
@@ -320,7 +323,7 @@ shn_status shn_trace_closest(const shn_grid* g, const shn_rays* rays, uint32_t n
   if (!counter) return set_error(g->ctx, SHN_ERR_OOM, "trace scratch");
   cudaMemsetAsync(counter, 0, 4, st);
   const GridView G = view_of(g);
-  const RaysView R{rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmax};
+  const RaysView R = view_rays(*rays, strides);
 #define SHN_LAUNCH_RAYS(K, S)                                                                   \
   {                                                                                             \
     static int blocks = persistent_blocks(k_trace_rays<K, false, S>, g->ctx->num_sms);          \
@@ -331,7 +334,7 @@ shn_status shn_trace_closest(const shn_grid* g, const shn_rays* rays, uint32_t n
   if (g->kind == SHN_GRID_UNIFORM) {
     if (g->stats) SHN_LAUNCH_RAYS(0, true)
     else
-      launch_flat_closest(G, *rays, n, counter, *hits, g->ctx->num_sms, st);
+      launch_flat_closest(G, R, n, counter, *hits, g->ctx->num_sms, st);
   } else {
     if (g->stats) SHN_LAUNCH_RAYS(1, true) else SHN_LAUNCH_RAYS(1, false)
   }
@@ -341,6 +344,11 @@ shn_status shn_trace_closest(const shn_grid* g, const shn_rays* rays, uint32_t n
 
 shn_status shn_trace_any(const shn_grid* g, const shn_rays* rays, uint32_t n, uint8_t* d_occluded,
                          void* stream) {
+  return shn_trace_any_strided(g, rays, nullptr, n, d_occluded, stream);
+}
+
+shn_status shn_trace_any_strided(const shn_grid* g, const shn_rays* rays, const shn_ray_strides* strides, uint32_t n,
+                                 uint8_t* d_occluded, void* stream) {
   if (!g || !rays || !d_occluded) return SHN_ERR_INVALID;
   if (!g->built) return set_error(g->ctx, SHN_ERR_NOT_BUILT, "grid not built");
   grid_fence(g, (cudaStream_t)stream);
@@ -353,7 +361,7 @@ shn_status shn_trace_any(const shn_grid* g, const shn_rays* rays, uint32_t n, ui
   if (!counter) return set_error(g->ctx, SHN_ERR_OOM, "trace scratch");
   cudaMemsetAsync(counter, 0, 4, st);
   const GridView G = view_of(g);
-  const RaysView R{rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmax};
+  const RaysView R = view_rays(*rays, strides);
 #define SHN_LAUNCH_ANY(K, S)                                                                    \
   {                                                                                             \
     static int blocks = persistent_blocks(k_trace_rays<K, true, S>, g->ctx->num_sms);           \
@@ -364,7 +372,7 @@ shn_status shn_trace_any(const shn_grid* g, const shn_rays* rays, uint32_t n, ui
   if (g->kind == SHN_GRID_UNIFORM) {
     if (g->stats) SHN_LAUNCH_ANY(0, true)
     else
-      launch_flat_any(G, *rays, n, counter, d_occluded, g->ctx->num_sms, st);
+      launch_flat_any(G, R, n, counter, d_occluded, g->ctx->num_sms, st);
   } else {
     if (g->stats) SHN_LAUNCH_ANY(1, true) else SHN_LAUNCH_ANY(1, false)
   }

@@ -85,3 +85,38 @@ def test_flat_traversal(gpu, tris, scale, res, rays):
         assert np.array_equal(a[keep], np.ascontiguousarray(x).view(np.uint32)), f"{name} differs from the oracle"
     ro = oracle.trace_any(og, org[keep], d[keep], tmax[keep])[0]
     assert np.array_equal(occ.cpu().numpy()[keep], np.asarray(ro).astype(np.uint8))
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+def test_strided_rays(gpu, kind):
+    """Rays read in place from sliced, transposed, repeated and padded arrays equal contiguous ones."""
+    import torch
+
+    import shinobi_b200 as shn
+    sc = scenes.uniform_soup(20000, seed=3)
+    g = shn.Grid().build(shn.FaceSoup(sc.vertices, sc.indices), shn.grid_params(kind))
+    b = oracle.bounds(sc.vertices, sc.indices)
+    org, d, tmax = [torch.from_numpy(x).cuda() for x in _rays(3001, b, seed=5)]
+    n = org.shape[0]
+    pad = torch.zeros(n, 8, device="cuda")
+    pad[:, 1:4], pad[:, 4:7], pad[:, 7] = org, d, tmax
+    one = org[1:2].expand(n, 3)
+    forms = [
+        (org, d, tmax, org, d, tmax),
+        (pad[:, 1:4], pad[:, 4:7], pad[:, 7], org, d, tmax),
+        (org.t().contiguous().t(), d.t().contiguous().t(), tmax, org, d, tmax),
+        (org[::2], d[::2], tmax[::2], org[::2].contiguous(), d[::2].contiguous(), tmax[::2].contiguous()),
+        (one, d, tmax[:1].expand(n), one.contiguous(), d, tmax[:1].expand(n).contiguous()),
+        (org, d, None, org, d, torch.full((n,), 3.4028234663852886e38, device="cuda")),
+    ]
+    for o, w, t, o2, w2, t2 in forms:
+        ref = shn.alloc_hits(o.shape[0])
+        rays, keep = shn.Grid._rays(o2, w2, t2)
+        import ctypes as C
+        h = ref.struct()
+        g.ctx.check(g.ctx.lib.shn_trace_closest(g.handle, C.byref(rays), o.shape[0], C.byref(h), shn._stream(None)), "")
+        got = g.trace_closest(o, w, t)
+        for a, x in ((got.tri, ref.tri), (got.t, ref.t), (got.u, ref.u), (got.v, ref.v)):
+            assert torch.equal(a.view(torch.int32), x.view(torch.int32))
+        if t is not None:
+            assert torch.equal(g.trace_any(o, w, t).bool(), ref.tri != -1)

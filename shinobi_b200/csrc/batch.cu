@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kBatchTraceBlock, kFlatBlocks) k_batch_trace(G
   __shared__ FlatWarp sm[kBatchTraceBlock / 32];
   flat_trace<ANY>(
       sm, BatchAcc{scenes, cells, refs_of(G)}, n, ou || ov, counter,
-      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t& scene) {
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t& scene, uint32_t&) {
         uint32_t lo = 0, hi = ns;
         while (hi - lo > 1) {
           const uint32_t mid = (lo + hi) >> 1;

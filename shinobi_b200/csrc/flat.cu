@@ -15,7 +15,7 @@ __global__ void __launch_bounds__(kCoopBlock, kFlatBlocks) k_flat_rays(const __g
   __shared__ FlatWarp sm[kCoopBlock / 32];
   flat_trace<ANY>(
       sm, FlatGrid{&G}, n, ou || ov, counter,
-      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) {
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&, uint32_t&) {
         R.ray(i, o, d, tmax);
       },
       [&](uint32_t i, const Hit& h, uint32_t) {
@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(kCoopBlock, kFlatBlocks) k_flat_camera(const _
   __shared__ FlatWarp sm[kCoopBlock / 32];
   flat_trace<false>(
       sm, FlatGrid{&G}, n, ou || ov, counter,
-      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) {
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&, uint32_t&) {
         o = cam.eye;
         d = primary_dir(cam, tile_pixel(cam, i), image_id);
         tmax = FLT_MAX;
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kCoopBlock, kFlatBlocks) k_flat_from_hits(cons
   __shared__ FlatWarp sm[kCoopBlock / 32];
   flat_trace<true>(
       sm, FlatGrid{&G}, (*d_m) * spp, false, counter,
-      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) { R.ray(i, o, d, tmax); },
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&, uint32_t&) { R.ray(i, o, d, tmax); },
       [&](uint32_t i, const Hit& h, uint32_t) { R.done(i, h); });
 }
 

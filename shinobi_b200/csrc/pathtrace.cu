@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kPtBlock, kFlatBlocks) k_pt_flat(const __grid_
   __shared__ FlatWarp sm[kPtBlock / 32];
   flat_trace<ANY>(
       sm, FlatGrid{&G}, *n, false, counter,
-      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&) { R.ray(i, o, d, tmax); },
+      [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&, uint32_t&) { R.ray(i, o, d, tmax); },
       [&](uint32_t i, const Hit& h, uint32_t) { R.done(i, h); });
 }
 

@@ -23,7 +23,7 @@
 #include <unordered_map>
 
 #include "internal.h"
-#include "trace_coop.cuh"
+#include "trace_flat.cuh"
 
 namespace shn {
 namespace {
@@ -45,18 +45,18 @@ struct ServeAcc {
   const ServeSeg* __restrict__ segs;
   SHN_D const Geom& geom(uint32_t s) const { return segs[s].g.g; }
   SHN_D const uint2* cells(uint32_t s) const { return segs[s].g.cells; }
-  SHN_D const uint2* leaves(uint32_t s) const { return segs[s].g.leaves; }
+  SHN_D uint32_t cell0(uint32_t) const { return 0u; }
   SHN_D Refs refs(uint32_t s) const { return refs_of(segs[s].g); }
 };
 
 // Rays are AoS records of 8 floats: ox, oy, oz, dx, dy, dz, tmax, unused.
-__global__ void __launch_bounds__(kServeBlock, 8) k_serve_trace(const ServeSeg* __restrict__ segs, uint32_t nseg,
+__global__ void __launch_bounds__(kServeBlock, 6) k_serve_trace(const ServeSeg* __restrict__ segs, uint32_t nseg,
                                                             const float4* __restrict__ rays, uint32_t n,
                                                             uint32_t* counter, uint32_t* __restrict__ otri,
                                                             float* __restrict__ ot) {
-  // incoherent request rays rarely share a cell range: no grouping
-  warp_trace_acc<0, false, false>(
-      ServeAcc{segs}, n, counter,
+  __shared__ FlatWarp sm[kServeBlock / 32];
+  flat_trace<false, true>(
+      sm, ServeAcc{segs}, n, false, counter,
       [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t& seg, uint32_t& anyhit) {
         uint32_t lo = 0, hi = nseg;
         while (hi - lo > 1) {
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kServeBlock, 8) k_serve_trace(const ServeSeg* 
         d = mk(a.w, b.x, b.y);
         tmax = b.z;
       },
-      [&](uint32_t i, const Hit& h, uint32_t, uint32_t, uint32_t) {
+      [&](uint32_t i, const Hit& h, uint32_t) {
         otri[i] = h.tri;
         ot[i] = h.t;
       });

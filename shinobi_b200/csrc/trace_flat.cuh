@@ -53,7 +53,7 @@ struct FlatWarp {
   float4 a[32];  // org, Sx
   float4 b[32];  // Sy, Sz, axis permutation, bound (the best t so far)
   float4 c[32];  // tMax, cell
-  float4 d[32];  // tDelta, direction signs and scene
+  float4 d[32];  // tDelta, direction signs (3 bits), any-hit flag, scene
   uint2 e[32];   // steps left in x and y | in z, cells ahead known to be empty
   uint32_t rid[32], best[32];
   unsigned long long key[32];         // least (t, cell of the window, triangle id) of the ranges under test
@@ -70,6 +70,12 @@ SHN_D unsigned long long flat_key(float t, uint32_t q, uint32_t id) {
   return ((unsigned long long)__float_as_uint(t) << 33) | ((unsigned long long)q << 30) | id;
 }
 SHN_D float flat_key_t(unsigned long long k) { return __uint_as_float((uint32_t)(k >> 33)); }
+
+// Key of an any-hit ray among closest-hit ones: its first hit in the order of
+// the cells and their references (fewer than 2^30).
+SHN_D unsigned long long flat_key_any(float t, uint32_t q, uint32_t ref) {
+  return ((unsigned long long)q << 61) | ((unsigned long long)ref << 31) | __float_as_uint(t);
+}
 
 enum : int { FLAT_MISS = 0, FLAT_RAY = 1, FLAT_GENERAL = 2 };
 
@@ -122,7 +128,7 @@ SHN_D void flat_axis(float gmin, float cs, int res, float org, float rcp, float 
 }
 
 SHN_D void flat_queue(const Geom& g, uint32_t cell0, V3 org, V3 dir, float tmax, V3 cell, uint32_t rid, uint32_t scene,
-                      FlatWarp& Q, uint32_t k) {
+                      uint32_t anyhit, FlatWarp& Q, uint32_t k) {
   const V3 rcp = divv(mk(1.f, 1.f, 1.f), dir);
   const RayWT w = wt_setup(org, dir);
   const uint32_t perm = (uint32_t)w.kx | ((uint32_t)w.ky << 2) | ((uint32_t)w.kz << 4);
@@ -137,7 +143,7 @@ SHN_D void flat_queue(const Geom& g, uint32_t cell0, V3 org, V3 dir, float tmax,
   const uint32_t idx = cell0 + (uint32_t)ix + (uint32_t)iy * (uint32_t)g.res[0] + (uint32_t)iz * (uint32_t)g.res[0] * (uint32_t)g.res[1];
   const uint32_t signs = (rcp.x > 0.f ? 1u : 0u) | (rcp.y > 0.f ? 2u : 0u) | (rcp.z > 0.f ? 4u : 0u);
   Q.c[k] = make_float4(tm.x, tm.y, tm.z, __uint_as_float(idx));
-  Q.d[k] = make_float4(dl.x, dl.y, dl.z, __uint_as_float(signs | scene << 3));
+  Q.d[k] = make_float4(dl.x, dl.y, dl.z, __uint_as_float(signs | (anyhit ? 8u : 0u) | scene << 4));
   Q.e[k] = make_uint2(lx | ly << 16, lz);
   Q.rid[k] = rid;
   Q.best[k] = kMiss;
@@ -146,10 +152,11 @@ SHN_D void flat_queue(const Geom& g, uint32_t cell0, V3 org, V3 dir, float tmax,
 // A ray whose walk does not start plainly: the general state machine, alone.
 template <bool ANY, bool IND>
 __device__ __noinline__ void flat_general(const Geom& g, const uint2* cells, const Refs& R, V3 org, V3 dir, float tmax,
-                                          Hit& h) {
+                                          uint32_t anyhit, Hit& h) {
   Lane L;
   uint32_t steps = 0, tests = 0;
   lane_init<0>(g, L, org, dir, tmax);
+  L.anyhit = anyhit;
   while (lane_advance<0, ANY>(g, cells, nullptr, L, steps)) lane_range<ANY, IND>(R, L, tests);
   lane_result(R, L, h);
 }
@@ -185,17 +192,20 @@ constexpr uint32_t kFlatLong = 63, kFlatHuge = 1u << 24;
 // The long ranges, listed from the end of W.own (lane and cell | length << 8,
 // first reference): per distinct range, each lane loads one reference of
 // every 32 and tests it against each waiting ray.
-template <bool ANY>
-SHN_D void flat_long(FlatWarp& W, const Refs& R, uint32_t count) {
+template <bool ANY, bool MIXED, class Acc>
+SHN_D void flat_long(FlatWarp& W, const Acc& acc, uint32_t count) {
   const int lane = threadIdx.x & 31;
   for (uint32_t k0 = 0; k0 < count; k0 += 32) {
     uint2 mine = make_uint2(0u, 0u);
     if (k0 + lane < count) mine = W.own[32 * kFlatAhead + 31 - (k0 + lane)];
+    const uint32_t mscene = MIXED ? __float_as_uint(W.d[mine.x & 31u].w) >> 4 : 0u;
     uint32_t todo = __ballot_sync(0xFFFFFFFFu, k0 + lane < count);
     while (todo) {
       const int j = __ffs(todo) - 1;
       const uint32_t b = __shfl_sync(0xFFFFFFFFu, mine.y, j), len = __shfl_sync(0xFFFFFFFFu, mine.x, j) >> 8;
-      const uint32_t rays = todo & __ballot_sync(0xFFFFFFFFu, mine.y == b && (mine.x >> 8) == len);
+      const uint32_t scene = __shfl_sync(0xFFFFFFFFu, mscene, j);
+      const Refs R = acc.refs(scene);
+      const uint32_t rays = todo & __ballot_sync(0xFFFFFFFFu, mine.y == b && (mine.x >> 8) == len && mscene == scene);
       todo &= ~rays;
       for (uint32_t i0 = 0; i0 < len; i0 += 32) {
         const bool in = i0 + lane < len;
@@ -208,18 +218,21 @@ SHN_D void flat_long(FlatWarp& W, const Refs& R, uint32_t count) {
           const float4 A = W.a[owner], B = W.b[owner];
           float t;
           if (in && wt_test_p<3, 3, 3>(f4v(A), A.w, B.x, B.y, p0, p1, p2, kEps, B.w, t, __float_as_uint(B.z)))
-            atomicMin(&W.key[owner], flat_key(t, slot >> 5, id));
+            atomicMin(&W.key[owner], MIXED && (__float_as_uint(W.d[owner].w) & 8u)
+                                         ? flat_key_any(t, slot >> 5, b + i0 + lane)
+                                         : flat_key(t, slot >> 5, id));
         }
       }
     }
   }
 }
 
-// Rays [0, n) from *counter (zeroed).  src(i, org, dir, tmax, scene) makes
-// ray i; sink(i, hit, scene) takes its result, whose u and v are only
-// computed if `uv`.  The accessor's scenes share one reference array of
-// fewer than kFlatMaxTris triangles.
-template <bool ANY, class Acc, class Src, class Sink>
+// Rays [0, n) from *counter (zeroed).  src(i, org, dir, tmax, scene, anyhit)
+// makes ray i; sink(i, hit, scene) takes its result, whose u and v are only
+// computed if `uv`.  Scenes have fewer than kFlatMaxTris triangles.  MIXED:
+// every scene has arrays of its own, and rays may be any-hit one by one
+// (otherwise the scenes share one array of cells and one of references).
+template <bool ANY, bool MIXED = false, class Acc, class Src, class Sink>
 SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint32_t* counter, Src&& src, Sink&& sink) {
   constexpr bool IND = true;
   static_assert(Acc::kIndirect, "triangles are read by id");
@@ -227,8 +240,8 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
   // rays reserved at a time, one reservation ahead of its use; fewer when there
   // are few rays for every warp
   const uint32_t grab = min(32u, max(1u, n / (4u * gridDim.x * (blockDim.x >> 5))));
-  const Refs R = acc.refs(0u);
-  const uint2* __restrict__ cells = acc.cells(0u);
+  const Refs R0 = MIXED ? Refs{} : acc.refs(0u);
+  const uint2* __restrict__ cells0 = MIXED ? nullptr : acc.cells(0u);
   FlatWarp& W = smem[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
@@ -255,11 +268,11 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
             w.Sx = A.w;
             w.Sy = B.x;
             w.Sz = B.y;
-            const float4* rec = R.src + 3 * (size_t)h.tri;
+            const float4* rec = (MIXED ? acc.refs(__float_as_uint(W.d[lane].w) >> 4).src : R0.src) + 3 * (size_t)h.tri;
             float t;
             wt_test(w, __ldg(rec), __ldg(rec + 1), __ldg(rec + 2), kEps, INFINITY, t, h.u, h.v);
           }
-          sink(W.rid[lane], h, __float_as_uint(W.d[lane].w) >> 3);
+          sink(W.rid[lane], h, __float_as_uint(W.d[lane].w) >> 4);
           fin = false;
         }
         while (true) {
@@ -272,10 +285,10 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
               const uint32_t i = W.wait[waiting + rank];
               V3 o, d, cell;
               float tmax;
-              uint32_t sc = 0;
-              src(i, o, d, tmax, sc);
+              uint32_t sc = 0, ah = 0;
+              src(i, o, d, tmax, sc, ah);
               flat_enter(acc.geom(sc), o, d, tmax, cell);
-              flat_queue(acc.geom(sc), acc.cell0(sc), o, d, tmax, cell, i, sc, W, lane);
+              flat_queue(acc.geom(sc), acc.cell0(sc), o, d, tmax, cell, i, sc, ah, W, lane);
               active = true;
             }
             __syncwarp();
@@ -293,8 +306,8 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
           if ((uint32_t)lane < grab && i < n) {
             V3 o, d, cell;
             float tmax;
-            uint32_t sc = 0;
-            src(i, o, d, tmax, sc);
+            uint32_t sc = 0, ah = 0;
+            src(i, o, d, tmax, sc, ah);
             what = flat_enter(acc.geom(sc), o, d, tmax, cell);
             if (what == FLAT_MISS) sink(i, Hit{tmax, kMiss, 0.f, 0.f}, sc);
           }
@@ -326,7 +339,8 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
           const uint2 E = W.e[lane];
           const float bound = W.b[lane].w;
           const uint32_t bits = __float_as_uint(D.w);
-          const Geom& g = acc.geom(bits >> 3);
+          const Geom& g = acc.geom(bits >> 4);
+          const uint2* __restrict__ cells = MIXED ? acc.cells(bits >> 4) : cells0;
           const int sx = bits & 1u ? 1 : -1, sy = bits & 2u ? g.res[0] : -g.res[0],
                     sz = bits & 4u ? g.res[0] * g.res[1] : -g.res[0] * g.res[1];
           float mx = C.x, my = C.y, mz = C.z;
@@ -398,11 +412,11 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
       }
       __syncwarp();
       // ---- test ------------------------------------------------------------------
-      if (nlong) flat_long<ANY>(W, R, nlong);
+      if (nlong) flat_long<ANY, MIXED>(W, acc, nlong);
       // The triangle ids of kFlatGroups groups of 32 references are loaded together.
       uint32_t started = 0;
       for (uint32_t j0 = 0; j0 < sum; j0 += 32u * kFlatGroups) {
-        uint32_t id[kFlatGroups], slot[kFlatGroups];
+        uint32_t id[kFlatGroups], slot[kFlatGroups], ref[kFlatGroups];
 #pragma unroll
         for (int k = 0; k < kFlatGroups; ++k) {
           slot[k] = ~0u;
@@ -416,7 +430,9 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
             if (j < sum) {
               const uint2 w = W.own[rank];
               slot[k] = w.x & 255u;
-              id[k] = __ldg(R.ridx + (j + w.y));
+              const uint32_t* ridx = MIXED ? acc.refs(__float_as_uint(W.d[w.x & 31u].w) >> 4).ridx : R0.ridx;
+              id[k] = __ldg(ridx + (j + w.y));
+              if (MIXED) ref[k] = j + w.y;
             }
           }
         }
@@ -424,10 +440,20 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
         for (int k = 0; k < kFlatGroups; ++k) {
           if (k != 0 && j0 + 32u * k >= sum) break;
           const uint32_t owner = slot[k] & 31u;
-          const float4* rec = R.src + 3 * (size_t)id[k];
+          // (a lane without a reference reads no ray's state: the place it would
+          // look at may hold none)
+          const bool mine = slot[k] != ~0u;
+          const uint32_t bits = MIXED && mine ? __float_as_uint(W.d[owner].w) : 0u;
+          const float4* rec = R0.src;
+          if (MIXED && mine) rec = acc.refs(bits >> 4).src;
+          rec += 3 * (size_t)(mine ? id[k] : 0u);
           int hit = 0;
           float t;
-          if (slot[k] != ~0u && (!ANY || W.key[owner] == ~0ull))
+          // (numbers go up with the cells and their references, so an any-hit
+          // ray's key from an earlier group stands)
+          const bool done = (ANY || (MIXED && (bits & 8u))) && W.key[owner] != ~0ull;
+          if (MIXED) __syncwarp();
+          if (mine && !done)
             hit = flat_test(W.a[owner], W.b[owner], __ldg(rec), __ldg(rec + 1), __ldg(rec + 2), t);
           if (__any_sync(0xFFFFFFFFu, hit == 2)) {
             if (hit == 2) {
@@ -436,7 +462,9 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
                                        __float_as_uint(B.z)) ? 1 : 0;
             }
           }
-          if (hit) atomicMin(&W.key[owner], flat_key(t, slot[k] >> 5, id[k]));
+          if (hit)
+            atomicMin(&W.key[owner],
+                      MIXED && (bits & 8u) ? flat_key_any(t, slot[k] >> 5, ref[k]) : flat_key(t, slot[k] >> 5, id[k]));
         }
       }
       __syncwarp();
@@ -450,7 +478,14 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
       if (active) {
         const unsigned long long k = some ? W.key[lane] : ~0ull;
         bool end = !on;
-        if (k != ~0ull) {
+        const uint32_t bits = MIXED ? __float_as_uint(W.d[lane].w) : 0u;
+        if (MIXED && (bits & 8u)) {
+          if (k != ~0ull) {
+            W.best[lane] = __ldg(acc.refs(bits >> 4).ridx + ((uint32_t)(k >> 31) & 0x3FFFFFFFu));
+            W.b[lane].w = __uint_as_float((uint32_t)k & 0x7FFFFFFFu);
+            end = true;
+          }
+        } else if (k != ~0ull) {
           const float t = flat_key_t(k);
           const uint32_t q = (uint32_t)(k >> 30) & 7u;
           float entry = -INFINITY;
@@ -477,10 +512,11 @@ SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint3
       const uint32_t i = W.general[k];
       V3 o, d;
       float tmax;
-      uint32_t sc = 0;
-      src(i, o, d, tmax, sc);
+      uint32_t sc = 0, ah = 0;
+      src(i, o, d, tmax, sc, ah);
       Hit h;
-      flat_general<ANY, IND>(acc.geom(sc), cells + acc.cell0(sc), R, o, d, tmax, h);
+      flat_general<ANY, IND>(acc.geom(sc), (MIXED ? acc.cells(sc) : cells0) + acc.cell0(sc), MIXED ? acc.refs(sc) : R0, o,
+                             d, tmax, ah, h);
       sink(i, h, sc);
     }
     __syncwarp();

@@ -120,3 +120,46 @@ def test_strided_rays(gpu, kind):
             assert torch.equal(a.view(torch.int32), x.view(torch.int32))
         if t is not None:
             assert torch.equal(g.trace_any(o, w, t).bool(), ref.tri != -1)
+
+
+@pytest.mark.parametrize("lambdas,rays", [((5.0, 0.5, 0.004), 1501), ((0.004, 0.02), 33), ((5.0,), 1)])
+def test_mixed_requests(gpu, lambdas, rays):
+    """Closest- and any-hit requests of several scenes in one launch, ranges of a few to thousands of
+    references: closest hits equal the oracle's bit for bit, any-hit answers its occlusion, and an any-hit
+    triangle is one the ray hits at the t given."""
+    import torch
+
+    import shinobi_b200 as shn
+    sv = shn.Server(num_slots=len(lambdas))
+    try:
+        reqs, want, keep = [], [], []
+        for k, lam in enumerate(lambdas):
+            sc = scenes.uniform_soup(4000 + 500 * k, seed=k + 1, offset_scale=0.02)
+            sv.load_scene(k, sc, lam)
+            b = oracle.bounds(sc.vertices, sc.indices)
+            og = oracle.build_uniform(sc.vertices, sc.indices, b, oracle.resolution(sc.num_triangles, b, lam, 1, 1))
+            for kind in (0, 1):
+                org, d, tmax = _rays(rays + 7 * k, b, seed=10 * k + kind)
+                r8 = torch.zeros(org.shape[0], 8).pin_memory()
+                r8[:, 0:3], r8[:, 3:6], r8[:, 6] = map(torch.from_numpy, (org, d, tmax))
+                tri = torch.zeros(org.shape[0], dtype=torch.int32).pin_memory()
+                t = torch.zeros(org.shape[0]).pin_memory()
+                reqs.append(sv.ray_request(kind, k, r8, tri, t))
+                keep.append(r8)
+                want.append((kind, sc, og, org, d, tmax, tri, t))
+        res = sv.run_schedule(reqs, np.zeros(len(reqs)))
+        assert not res.any()
+        for kind, sc, og, org, d, tmax, tri, t in want:
+            tri, t = tri.numpy().view(np.uint32), t.numpy()
+            if kind == 0:
+                rt, rtt = oracle.trace_closest(og, org, d, tmax)[:2]
+                assert np.array_equal(tri, rt) and np.array_equal(t.view(np.uint32), rtt.view(np.uint32))
+            else:
+                occ = np.asarray(oracle.trace_any(og, org, d, tmax)[0]).astype(bool)
+                hit = tri != shn.SHN_MISS
+                assert np.array_equal(hit, occ)
+                t64 = oracle.t_fp64(sc.vertices, sc.indices, tri, org, d)
+                near = hit & (np.abs(org).max(1) < 10.0)  # distant origins: t carries their rounding
+                assert np.all(np.abs(t[near] - t64[near]) <= 1e-4 * np.maximum(1.0, np.abs(t64[near])))
+    finally:
+        sv.close()

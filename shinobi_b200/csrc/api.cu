@@ -453,7 +453,7 @@ shn_status shn_grid_export(const shn_grid* g, uint32_t* cells, uint32_t* leaves,
       if (leaves[2 * i] == leaves[2 * i + 1]) leaves[2 * i] = leaves[2 * i + 1] = 0;
   }
   if (e == cudaSuccess && g->spatial) {
-    // a two-level grid was built on the triangles in Morton order: the
+    // a two-level grid was built on the triangles in Hilbert order: the
     // references of a leaf are in that order and the pairs' low words are
     // positions in it; both are put back in (cell, triangle id) order
     if (indices && g->num_refs) {

@@ -74,7 +74,7 @@ struct shn_grid {
   uint32_t* indices = nullptr;  // tri id per reference
   float4* rtri = nullptr;       // two-level: 3*num_refs: reference-ordered v0[], v1[], v2[]
   uint64_t* top_pairs = nullptr;  // two-level: sorted top pairs; uniform: sorted pairs
-  // two-level grids: the build runs on the triangles in Morton order (perm_tri,
+  // two-level grids: the build runs on the triangles in Hilbert order (perm_tri,
   // w = original id), so the pairs' low words are positions in that order;
   // boxes of every 32 references (cbox) and every 1024 (sbox) of rtri, two
   // float4 (min, max) each, let the traversal skip blocks a ray cannot hit

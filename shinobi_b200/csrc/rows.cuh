@@ -133,6 +133,12 @@ SHN_HD int class_at(const Unit& U, int r, float c, float tu, float tv) {
   return pass ? 0 : (d > 0.f ? 1 : -1);
 }
 
+// Rows of at most this many cells are tested cell by cell, without branches
+// between them: the search below keeps 20 of 32 lanes active in the count.
+// 64-scene batch 2.78 -> 2.70 ms, rebuild of a 4.2M-triangle soup 1.61 -> 1.58
+// ms; 3, 4 and 8 cells: 2.75, 2.75, 2.72 and 1.58, 1.58, 1.61 ms.
+constexpr uint32_t kShortRow = 6;
+
 SHN_HD uint32_t clamp_index(float x, uint32_t lo, uint32_t hi1) {
   const float c = fminf(fmaxf(x, (float)lo), (float)hi1);  // NaN -> lo
   uint32_t i = (uint32_t)c;
@@ -150,6 +156,28 @@ SHN_HD void row_interval(const Unit& U, uint32_t j, uint32_t& f, uint32_t& e) {
   const uint32_t lo = U.lo[r], hi1 = U.lo[r] + U.span[r];  // [lo, hi1)
   const float s = U.s[r];
   const float c0 = ((((float)lo * s + U.o[r]) + s * 0.5f) - s) + s;  // centre of lo
+  if (U.span[r] <= kShortRow) {
+    // the passing cells are one interval: its ends are the first and last one
+    const float nr = U.n[r], ar = U.a[r];
+    const float h0 = U.s[0] * 0.5f + kEps, h1 = U.s[1] * 0.5f + kEps, h2 = U.s[2] * 0.5f + kEps;
+    float c = c0;
+    uint32_t m = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kShortRow; ++k) {
+      const float d = combine(r, (c - ar) * nr, tu, tv);
+      const bool pass = fabsf(U.n[0] * d) <= h0 && fabsf(U.n[1] * d) <= h1 && fabsf(U.n[2] * d) <= h2;
+      if (pass && lo + k < hi1) m |= 1u << k;
+      c += s;
+    }
+    f = e = lo;
+#pragma unroll
+    for (uint32_t k = kShortRow; k-- > 0;)
+      if ((m >> k) & 1u) f = lo + k;
+#pragma unroll
+    for (uint32_t k = 0; k < kShortRow; ++k)
+      if ((m >> k) & 1u) e = lo + k + 1u;
+    return;
+  }
   const float nr = U.n[r];
   if (!(nr > 0.f) && !(nr < 0.f)) {  // the class is the same along the whole row
     if (class_at(U, r, c0, tu, tv) == 0) { f = lo; e = hi1; }

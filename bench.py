@@ -544,7 +544,7 @@ def run_shinobi(args):
         parity = frame_parity(cpu.pop("oracle_sample"), hits, ao, direct)
     # dominant kernel: the longer of the two trace kernels
     if ao_ms >= prim_ms:
-        kname = "k_trace_direct<two-level>" if direct else "k_trace_ao<two-level>"
+        kname = "k_trace_from_hits<two-level, DiRays>" if direct else "k_trace_from_hits<two-level, AoRays>"
         kms, ksteps, ktests = ao_ms, ao_steps, ao_tests
     else:
         kname, kms, ksteps, ktests = "k_trace_camera<two-level>", prim_ms, prim_steps, prim_tests
@@ -668,9 +668,9 @@ def launches_per_step(P, R, C0, L):
         return 1 + min(p8, p9)
     build = (2 + 1 + sort_launches(P, C0) + 1      # count + scan, emit, sort, top ranges
              + 1 + 2 + 1 + sort_launches(R, L) + 1)  # leaf cells scan, leaf count + scan, emit, sort, ranges
-    # Morton order of the triangles (keys, two 4-pass sorts, second keys, permute)
+    # Hilbert order of the triangles (keys, two 3-pass sorts, second keys, permute)
     # and the boxes per 32 and per 1024 references
-    spatial = 1 + 2 * (2 + 4) + 1 + 1 + (2 if R else 0) + 3   # + the three leaf-distance passes
+    spatial = 1 + 2 * (2 + 3) + 1 + 1 + (2 if R else 0) + 3   # + the three leaf-distance passes
     return build + spatial + 1 + 3                     # primary; compact + trace + finalize (AO or shading)
 
 

@@ -1094,15 +1094,15 @@ shn_status ensure_buf(shn_grid* g, DevBuf& b, size_t bytes, cudaStream_t st) {
 }
 
 // Room for the rows of n items in key buffer `buf`, which the sort does not
-// need before the emission has read them: kRowsPerItem per item (the buffer
-// ends up about as large for the keys), or what the buffer has.  0 when the
-// budget or the device has no room for them: the emission then finds the rows
-// again.
+// need before the emission has read them: what the buffer has and, in a
+// context without a memory budget, at least kRowsPerItem per item (the buffer
+// ends up about as large for the keys).  Under a budget nothing is allocated
+// for rows, so a build needs no more memory than its keys do.
 constexpr uint64_t kRowsPerItem = 6;
 
 uint64_t rows_room(shn_grid* g, int buf, uint64_t n, cudaStream_t st) {
   const size_t want = std::min<uint64_t>(n * kRowsPerItem, 1ull << 30) * sizeof(uint2);
-  if (g->keys[buf].bytes < want && ensure_buf(g, g->keys[buf], want, st) != SHN_OK) return 0;
+  if (g->keys[buf].bytes < want && g->ctx->budget == 0 && ensure_buf(g, g->keys[buf], want, st) != SHN_OK) return 0;
   return g->keys[buf].bytes / sizeof(uint2);
 }
 

@@ -1,7 +1,8 @@
 """Key emission from the rows kept by the count: groups whose rows fit, groups
 whose rows do not (large triangles exceed the room of a first build), both in
 one build, one-item and ragged last groups.  Grids must equal the oracle's, on
-a first build and on the next ones, whose buffers have grown."""
+a first build and on the next ones, whose buffers have grown; under a memory
+budget a first build keeps no rows."""
 import numpy as np
 import pytest
 
@@ -27,13 +28,11 @@ def _mixed(n, small, large, every):
     (5000, 0.01, 0.02, 2, (50, 51, 52)),    # all fit
     (70, 0.5, 0.5, 1, (2048, 2, 2)),        # the longest rows
 ])
-@pytest.mark.parametrize("kind", [0, 1])
-def test_kept_rows(gpu, n, small, large, every, res, kind):
+@pytest.mark.parametrize("kind,budget", [(0, False), (1, False), (0, True), (1, True)])
+def test_kept_rows(gpu, n, small, large, every, res, kind, budget):
     import shinobi_b200 as shn
     v, i = _mixed(n, small, large, every)
     b = oracle.bounds(v, i)
-    soup = shn.FaceSoup(v, i)
-    g = shn.Grid()
     if kind == 0:
         p = shn.grid_params(shn.SHN_GRID_UNIFORM, res=res)
         og = oracle.build_uniform(v, i, b, np.array(res, np.int32))
@@ -41,6 +40,9 @@ def test_kept_rows(gpu, n, small, large, every, res, kind):
         res = tuple(max(2, r // 8) for r in res)
         p = shn.grid_params(shn.SHN_GRID_TWO_LEVEL, lambda_leaf=4.0, leaf_threshold=2, res=res)
         og = oracle.build_two_level(v, i, b, np.array(res, np.int32), 4.0, 2)
+    ctx = shn.Context(0, 8 << 30) if budget else gpu
+    soup = shn.FaceSoup(v, i, ctx=ctx)
+    g = shn.Grid(ctx=ctx)
     for _ in range(3):
         g.build(soup, p)
         ex = g.export()

@@ -44,12 +44,19 @@ constexpr int kFlatBlocks = 7;
 constexpr int kFlatGroups = 2;
 
 // Cells a lane walks per step of the warp, their ranges in flight together.
-constexpr int kFlatAhead = 6;
+// Calls of fewer rays than the device has lanes for (148 SMs x 7 blocks x 128)
+// wait for one ray's chain of windows and take longer ones: 200,000-triangle
+// soup, 1,021 / 16,000 / 64,000 / 130,000 rays 56 -> 50, 117 -> 86, 173 -> 159 and
+// 186 -> 170 us; from 200,000 rays on the shorter ones with a block more per SM
+// are as fast or faster (4.0M rays: 0.92 against 0.94 ms).
+constexpr int kFlatAhead = 6, kFlatAheadFew = 8;
+constexpr uint32_t kFlatFew = 1u << 17;
 
 // Shared memory of one warp.  The rays live here, not in registers: the walk
 // loads and stores what it needs, so that the tests have the registers.  Every
 // kilobyte less leaves L1 room for lines in flight.
-struct FlatWarp {
+template <int K>
+struct FlatWarpOf {
   float4 a[32];  // org, Sx
   float4 b[32];  // Sy, Sz, axis permutation, bound (the best t so far)
   float4 c[32];  // tMax, cell
@@ -57,15 +64,17 @@ struct FlatWarp {
   uint2 e[32];   // steps left in x and y | in z, cells ahead known to be empty
   uint32_t rid[32], best[32];
   unsigned long long key[32];         // least (t, cell of the window, triangle id) of the ranges under test
-  uint2 own[32 * kFlatAhead + 32];    // range under test: lane and cell | first number << 8, first reference - first number
+  uint2 own[32 * K + 32];    // range under test: lane and cell | first number << 8, first reference - first number
   uint32_t wait[32];                  // rays that meet the grid and have no lane yet
   uint32_t general[96];               // < 32 when rays are taken, and at most 32 + 31 more on their way
 };
 
+using FlatWarp = FlatWarpOf<kFlatAhead>;
+
 // Key of a candidate: t (positive: 31 bits), cell of the window (3 bits),
 // triangle id (30 bits).
 constexpr uint32_t kFlatMaxTris = 1u << 30;
-static_assert(kFlatAhead <= 8, "three bits of the key");
+static_assert(kFlatAhead <= 8 && kFlatAheadFew <= 8, "three bits of the key");
 SHN_D unsigned long long flat_key(float t, uint32_t q, uint32_t id) {
   return ((unsigned long long)__float_as_uint(t) << 33) | ((unsigned long long)q << 30) | id;
 }
@@ -127,8 +136,9 @@ SHN_D void flat_axis(float gmin, float cs, int res, float org, float rcp, float 
   left = (uint32_t)(up ? res - 1 - i : i);
 }
 
+template <int K>
 SHN_D void flat_queue(const Geom& g, uint32_t cell0, V3 org, V3 dir, float tmax, V3 cell, uint32_t rid, uint32_t scene,
-                      uint32_t anyhit, FlatWarp& Q, uint32_t k) {
+                      uint32_t anyhit, FlatWarpOf<K>& Q, uint32_t k) {
   const V3 rcp = divv(mk(1.f, 1.f, 1.f), dir);
   const RayWT w = wt_setup(org, dir);
   const uint32_t perm = (uint32_t)w.kx | ((uint32_t)w.ky << 2) | ((uint32_t)w.kz << 4);
@@ -192,12 +202,12 @@ constexpr uint32_t kFlatLong = 63, kFlatHuge = 1u << 24;
 // The long ranges, listed from the end of W.own (lane and cell | length << 8,
 // first reference): per distinct range, each lane loads one reference of
 // every 32 and tests it against each waiting ray.
-template <bool ANY, bool MIXED, class Acc>
-SHN_D void flat_long(FlatWarp& W, const Acc& acc, uint32_t count) {
+template <bool ANY, bool MIXED, int K, class Acc>
+SHN_D void flat_long(FlatWarpOf<K>& W, const Acc& acc, uint32_t count) {
   const int lane = threadIdx.x & 31;
   for (uint32_t k0 = 0; k0 < count; k0 += 32) {
     uint2 mine = make_uint2(0u, 0u);
-    if (k0 + lane < count) mine = W.own[32 * kFlatAhead + 31 - (k0 + lane)];
+    if (k0 + lane < count) mine = W.own[32 * K + 31 - (k0 + lane)];
     const uint32_t mscene = MIXED ? __float_as_uint(W.d[mine.x & 31u].w) >> 4 : 0u;
     uint32_t todo = __ballot_sync(0xFFFFFFFFu, k0 + lane < count);
     while (todo) {
@@ -213,7 +223,7 @@ SHN_D void flat_long(FlatWarp& W, const Acc& acc, uint32_t count) {
         const float4* rec = R.src + 3 * (size_t)id;
         const float4 p0 = __ldg(rec), p1 = __ldg(rec + 1), p2 = __ldg(rec + 2);
         for (uint32_t m = rays; m; m &= m - 1) {
-          const uint32_t slot = W.own[32 * kFlatAhead + 31 - (k0 + __ffs(m) - 1)].x & 255u, owner = slot & 31u;
+          const uint32_t slot = W.own[32 * K + 31 - (k0 + __ffs(m) - 1)].x & 255u, owner = slot & 31u;
           if (ANY && *reinterpret_cast<volatile unsigned long long*>(&W.key[owner]) != ~0ull) continue;
           const float4 A = W.a[owner], B = W.b[owner];
           float t;
@@ -232,17 +242,16 @@ SHN_D void flat_long(FlatWarp& W, const Acc& acc, uint32_t count) {
 // computed if `uv`.  Scenes have fewer than kFlatMaxTris triangles.  MIXED:
 // every scene has arrays of its own, and rays may be any-hit one by one
 // (otherwise the scenes share one array of cells and one of references).
-template <bool ANY, bool MIXED = false, class Acc, class Src, class Sink>
-SHN_D void flat_trace(FlatWarp* smem, const Acc& acc, uint32_t n, bool uv, uint32_t* counter, Src&& src, Sink&& sink) {
+template <bool ANY, bool MIXED = false, int K, class Acc, class Src, class Sink>
+SHN_D void flat_trace(FlatWarpOf<K>* smem, const Acc& acc, uint32_t n, bool uv, uint32_t* counter, Src&& src, Sink&& sink) {
   constexpr bool IND = true;
   static_assert(Acc::kIndirect, "triangles are read by id");
-  constexpr int K = kFlatAhead;
   // rays reserved at a time, one reservation ahead of its use; fewer when there
   // are few rays for every warp
   const uint32_t grab = min(32u, max(1u, n / (4u * gridDim.x * (blockDim.x >> 5))));
   const Refs R0 = MIXED ? Refs{} : acc.refs(0u);
   const uint2* __restrict__ cells0 = MIXED ? nullptr : acc.cells(0u);
-  FlatWarp& W = smem[threadIdx.x >> 5];
+  FlatWarpOf<K>& W = smem[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
   uint32_t next = 0;  // lane 0: first ray of the reservation ahead

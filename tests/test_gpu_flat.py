@@ -45,6 +45,8 @@ def _rays(n, b, seed):
     (3000, 0.02, (1, 40, 3), 1000),       # up to ~100 references in a cell
     (20000, 0.01, (2, 2, 2), 777),        # thousands of references in a cell
     (20000, 0.01, (40, 41, 39), 20011),
+    (20000, 0.01, (40, 41, 39), 131071),  # either side of the window lengths' limit
+    (20000, 0.01, (40, 41, 39), 131072),
     (40000, 0.004, (163, 162, 161), 30001),  # above the size with empty-cell distances
     (2000, 0.01, (2048, 2, 3), 5003),     # the longest axis
 ])

@@ -253,8 +253,11 @@ shn_status shn_grid_create(shn_ctx* ctx, shn_grid** out);
  * device wait gave up before those points.  The last stage (sort, ranges and
  * what follows) runs asynchronously on stream: traces, exports and info calls
  * of the grid, on any stream, are ordered after it, and a wait that gives up
- * there is reported by shn_grid_sync_status.  Traces of the grid read the
- * scene's triangles (hit records, normals), so the scene must outlive them. */
+ * there is reported by shn_grid_sync_status.  Traces of the grid test its own
+ * copy of the triangles: until the next build, new vertices of the scene do
+ * not change what is hit or where.  The u and v of hits and the shading
+ * normals are computed from the scene's triangles as they are then, so the
+ * scene must outlive the traces. */
 shn_status shn_grid_build(shn_grid* g, const shn_scene* s, const shn_grid_params* p, void* stream);
 shn_status shn_grid_get_info(const shn_grid* g, shn_grid_info* out);
 /* Copies the grid to host buffers (any may be NULL): cells = 2*num_cells

@@ -250,7 +250,7 @@ void enqueue_build(shn_batch* b, cudaStream_t st) {
 GridView batch_view(const shn_batch* b) {
   GridView v{};
   v.kind = 0;
-  v.src = b->tri;
+  v.src = v.rec = b->tri;
   v.ridx = b->indices;
   return v;
 }

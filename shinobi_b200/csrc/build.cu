@@ -49,6 +49,13 @@ SHN_D void load_tri(const TriArr& t, uint32_t i, V3& a, V3& b, V3& c) {
   c = f4v(__ldg(r + 2));
 }
 
+// The record itself, for a grid that keeps its own.
+SHN_D void keep_record(const TriArr& t, uint32_t i, float4* out) {
+  const float4* r = t.p + 3 * (size_t)i;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) out[3 * (size_t)i + k] = __ldg(r + k);
+}
+
 SHN_D void tri_bounds(V3 a, V3 b, V3 c, V3& bmin, V3& bmax) {
   bmin = mk(FLT_MAX, FLT_MAX, FLT_MAX);
   bmax = mk(-FLT_MAX, -FLT_MAX, -FLT_MAX);
@@ -175,6 +182,7 @@ SHN_D void leaf_unit(V3 a, V3 b, V3 c, const Geom& g, uint32_t topCell, uint32_t
 struct TopMaker {
   TriArr tri;
   Geom g;
+  float4* keep = nullptr;  // where the count leaves the records (uniform grids)
   SHN_D void item(uint32_t t, uint32_t& id, uint32_t stride[2]) const {
     id = t;
     stride[0] = (uint32_t)g.resf.x;
@@ -183,6 +191,7 @@ struct TopMaker {
   SHN_D bool operator()(uint32_t t, Unit& U) const {
     V3 a, b, c;
     load_tri(tri, t, a, b, c);
+    if (keep) keep_record(tri, t, keep);
     top_unit(a, b, c, g, t, 0u, U);
     return true;
   }
@@ -386,8 +395,9 @@ SHN_D void sat_cells(const TriArr& tri, const Geom& g, uint32_t t, F&& emit) {
   }
 }
 
-__global__ void k_count_sat(TriArr tri, uint32_t n, Geom g, uint32_t* __restrict__ counts) {
+__global__ void k_count_sat(TriArr tri, uint32_t n, Geom g, uint32_t* __restrict__ counts, float4* keep) {
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    if (keep) keep_record(tri, t, keep);
     uint32_t k = 0;
     sat_cells(tri, g, t, [&](uint32_t) { ++k; });
     counts[t] = k;
@@ -1017,12 +1027,13 @@ void launch_emit(Maker mk, uint32_t n, const uint32_t* offs, void* ws, const uin
 }
 
 // The counts and offsets of the precise insertion (as launch_counts).
-void launch_counts_sat(TriArr tri, Geom g, uint32_t n, uint32_t* offs, void* ws, uint32_t* err, cudaStream_t st) {
+void launch_counts_sat(TriArr tri, Geom g, float4* keep, uint32_t n, uint32_t* offs, void* ws, uint32_t* err,
+                       cudaStream_t st) {
   const size_t tiles = ((size_t)n + kScanTile - 1) / kScanTile;
   uint64_t* status = (uint64_t*)ws;
   cudaMemsetAsync(status, 0, (tiles + 2) * 8, st);
   uint32_t* ticket = (uint32_t*)(status + tiles + 1);
-  k_count_sat<<<grid_for(n, 128, 148 * 16), 128, 0, st>>>(tri, n, g, offs);
+  k_count_sat<<<grid_for(n, 128, 148 * 16), 128, 0, st>>>(tri, n, g, offs, keep);
   k_scan_inplace<<<(unsigned)tiles, kScanBlock, 0, st>>>(offs, n, LookbackState{status, ticket, err});
 }
 
@@ -1223,6 +1234,18 @@ shn_status build_grid(shn_grid* g, const shn_scene* s, const shn_grid_params* p,
     tri = TriArr{(const float4*)g->perm_tri.ptr};
   }
 
+  // ---- uniform: the grid's own records --------------------------------------------
+  // Traces test the triangles that the cells were made of, whatever becomes of
+  // the scene's vertices, as on a two-level grid; a copy by id (not by
+  // reference: a ninth of that on a soup, and it stays in L2), written by the
+  // count, which has the records at hand.  A view's triangles are its owner's.
+  float4* keep = nullptr;
+  g->rec = s->ids;
+  if (p->kind == SHN_GRID_UNIFORM && !s->ids) {
+    if ((rc = ensure(g, (void**)&g->rtri, &g->cap_rtri, (size_t)std::max<uint32_t>(nt, 1) * 48, st))) return rc;
+    g->rec = keep = g->rtri;
+  }
+
   // ---- counts + offsets ------------------------------------------------------
   if ((rc = ensure_buf(g, g->offs_tri, ((size_t)nt + 1) * 4, st))) return rc;
   uint32_t* offs = (uint32_t*)g->offs_tri.ptr;
@@ -1231,8 +1254,8 @@ shn_status build_grid(shn_grid* g, const shn_scene* s, const shn_grid_params* p,
   if (nt) {
     if ((rc = ensure_buf(g, g->scan, counts_bytes(nt), st))) return rc;
     if (!sat) row_cap = rows_room(g, 1, nt, st);
-    if (sat) launch_counts_sat(tri, g->geom, nt, offs, g->scan.ptr, g->d_err, st);
-    else launch_counts(TopMaker{tri, g->geom}, nt, offs, g->scan.ptr, (uint2*)g->keys[1].ptr, row_cap, g->d_err, st);
+    if (sat) launch_counts_sat(tri, g->geom, keep, nt, offs, g->scan.ptr, g->d_err, st);
+    else launch_counts(TopMaker{tri, g->geom, keep}, nt, offs, g->scan.ptr, (uint2*)g->keys[1].ptr, row_cap, g->d_err, st);
     const unsigned long long* next = row_store(g->scan.ptr, nt, nullptr, 0).next;
     const uint32_t* src[3] = {offs + nt, (const uint32_t*)next, (const uint32_t*)next + 1};
     uint32_t got[3] = {0, 0, 0};
@@ -1268,8 +1291,7 @@ shn_status build_grid(shn_grid* g, const shn_scene* s, const shn_grid_params* p,
   if (p->kind == SHN_GRID_UNIFORM) {
     if ((rc = ensure(g, (void**)&g->indices, &g->cap_refs, (size_t)std::max<uint32_t>(P, 1) * 4, st))) return rc;
     // no reference-ordered triangle copy: traces read a reference's triangle
-    // through indices[] (the records are a ninth of the copy on a soup, and stay
-    // in L2), and the ids count from the start of the scene's array
+    // through indices[], whose ids count from the start of the array that rec is
     launch_cell_ranges(sortedTop, P, C, g->cells, g->indices, s->ids ? (uint32_t)((s->tri - s->ids) / 3) : 0u, st);
     g->cell_dist = C >= kCellDistMin;
     if (g->cell_dist) {

@@ -72,7 +72,9 @@ struct shn_grid {
   uint2* cells = nullptr;       // uniform ranges / two-level cell words
   uint2* leaves = nullptr;      // two-level leaf ranges
   uint32_t* indices = nullptr;  // tri id per reference
-  float4* rtri = nullptr;       // two-level: 3*num_refs: reference-ordered v0[], v1[], v2[]
+  // two-level: 3*num_refs: reference-ordered v0[], v1[], v2[]; uniform: the
+  // scene's 48-byte records as they were at the build, by triangle id
+  float4* rtri = nullptr;
   uint64_t* top_pairs = nullptr;  // two-level: sorted top pairs; uniform: sorted pairs
   // two-level grids: the build runs on the triangles in Hilbert order (perm_tri,
   // w = original id), so the pairs' low words are positions in that order;
@@ -104,6 +106,9 @@ struct shn_grid {
   // scene the grid was built over (triangles by id, for shading / AO frames)
   const float4* src_tri = nullptr;
   uint32_t src_nt = 0;
+  // uniform: the records that traces test, by the ids of indices[] (rtri, or
+  // the owner's array of a view)
+  const float4* rec = nullptr;
   // optional device counters {cell visits, triangle tests} of the stats kernels
   unsigned long long* stats = nullptr;
 };

@@ -261,6 +261,7 @@ GridView view_of(const shn_grid* g) {
   v.src = g->src_tri;
   if (g->kind == SHN_GRID_UNIFORM) {
     v.ridx = g->indices;
+    v.rec = g->rec;
   } else {
     v.rv0 = g->rtri;
     v.rv1 = g->rtri + g->num_refs;

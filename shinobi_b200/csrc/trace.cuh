@@ -11,8 +11,8 @@
 //
 // Two-level grids keep a reference-ordered SoA float4 copy of the triangles
 // (v0[ref], v1[ref], v2[ref]; v0.w carries the triangle id), so a leaf's
-// candidates are contiguous; uniform grids read the scene's records through
-// indices[].
+// candidates are contiguous; uniform grids keep a copy of the scene's records
+// and read them through indices[].
 #pragma once
 #include "common.cuh"
 
@@ -26,15 +26,17 @@ struct GridView {
   const float4* __restrict__ rv0;
   const float4* __restrict__ rv1;
   const float4* __restrict__ rv2;
-  // the scene's triangle records (48 bytes: v0 with the id in w, v1, v2),
-  // indexed by the id that rv0[].w holds
+  // the scene's triangle records as they are now (48 bytes: v0 with the id in
+  // w, v1, v2), indexed by the id that rv0[].w holds: for u and v
   const float4* __restrict__ src;
   // boxes (min, max) of references [32k, 32k + 32) and [1024s, 1024s + 1024)
   // of rv*, or null (no culling)
   const float4* __restrict__ cbox;
   const float4* __restrict__ sbox;
-  // when not null: no reference-ordered copy; reference i is src[3 * ridx[i]]
+  // when not null: no reference-ordered copy; reference i is rec[3 * ridx[i]],
+  // rec the records as they were at the build
   const uint32_t* __restrict__ ridx;
+  const float4* __restrict__ rec;
 };
 
 struct Hit {

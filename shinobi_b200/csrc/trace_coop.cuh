@@ -43,16 +43,17 @@ struct Refs {
   const float4* __restrict__ src;
   const float4* __restrict__ cbox;  // block boxes (see GridView), or null
   const float4* __restrict__ sbox;
-  const uint32_t* __restrict__ ridx;  // not null: reference i is src[3 * ridx[i]] (no rv*)
+  const uint32_t* __restrict__ ridx;  // not null: reference i is rec[3 * ridx[i]] (no rv*)
+  const float4* __restrict__ rec;
 };
-SHN_D Refs refs_of(const GridView& G) { return Refs{G.rv0, G.rv1, G.rv2, G.src, G.cbox, G.sbox, G.ridx}; }
+SHN_D Refs refs_of(const GridView& G) { return Refs{G.rv0, G.rv1, G.rv2, G.src, G.cbox, G.sbox, G.ridx, G.rec}; }
 
 // Triangle of reference i: from the reference-ordered arrays, or (IND: grids
 // that keep no reference-ordered copy) through the reference's triangle id.
 template <bool IND>
 SHN_D void ref_load(const Refs& G, uint32_t i, float4& p0, float4& p1, float4& p2) {
   if (IND) {
-    const float4* r = G.src + 3 * (size_t)__ldg(G.ridx + i);
+    const float4* r = G.rec + 3 * (size_t)__ldg(G.ridx + i);
     p0 = __ldg(r);
     p1 = __ldg(r + 1);
     p2 = __ldg(r + 2);

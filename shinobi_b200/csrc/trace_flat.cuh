@@ -220,7 +220,7 @@ SHN_D void flat_long(FlatWarpOf<K>& W, const Acc& acc, uint32_t count) {
       for (uint32_t i0 = 0; i0 < len; i0 += 32) {
         const bool in = i0 + lane < len;
         const uint32_t id = in ? __ldg(R.ridx + (b + i0 + lane)) : 0u;
-        const float4* rec = R.src + 3 * (size_t)id;
+        const float4* rec = R.rec + 3 * (size_t)id;
         const float4 p0 = __ldg(rec), p1 = __ldg(rec + 1), p2 = __ldg(rec + 2);
         for (uint32_t m = rays; m; m &= m - 1) {
           const uint32_t slot = W.own[32 * K + 31 - (k0 + __ffs(m) - 1)].x & 255u, owner = slot & 31u;
@@ -453,8 +453,8 @@ SHN_D void flat_trace(FlatWarpOf<K>* smem, const Acc& acc, uint32_t n, bool uv, 
           // look at may hold none)
           const bool mine = slot[k] != ~0u;
           const uint32_t bits = MIXED && mine ? __float_as_uint(W.d[owner].w) : 0u;
-          const float4* rec = R0.src;
-          if (MIXED && mine) rec = acc.refs(bits >> 4).src;
+          const float4* rec = R0.rec;
+          if (MIXED && mine) rec = acc.refs(bits >> 4).rec;
           rec += 3 * (size_t)(mine ? id[k] : 0u);
           int hit = 0;
           float t;

@@ -80,8 +80,11 @@ SHN_D unsigned long long flat_key(float t, uint32_t q, uint32_t id) {
 }
 SHN_D float flat_key_t(unsigned long long k) { return __uint_as_float((uint32_t)(k >> 33)); }
 
-// Key of an any-hit ray among closest-hit ones: its first hit in the order of
-// the cells and their references (fewer than 2^30).
+// Key of an any-hit ray among closest-hit ones: the first of its candidates in
+// the order of the cells and their references (fewer than 2^30).  A range's
+// candidate is that of warp_trace: the first hit of a short range, and of a
+// long one the nearest hit (t, triangle id) among the first 32 references that
+// hold any.
 SHN_D unsigned long long flat_key_any(float t, uint32_t q, uint32_t ref) {
   return ((unsigned long long)q << 61) | ((unsigned long long)ref << 31) | __float_as_uint(t);
 }
@@ -167,7 +170,19 @@ __device__ __noinline__ void flat_general(const Geom& g, const uint2* cells, con
   uint32_t steps = 0, tests = 0;
   lane_init<0>(g, L, org, dir, tmax);
   L.anyhit = anyhit;
-  while (lane_advance<0, ANY>(g, cells, nullptr, L, steps)) lane_range<ANY, IND>(R, L, tests);
+  while (lane_advance<0, ANY>(g, cells, nullptr, L, steps)) {
+    if (!ANY && L.anyhit && L.e - L.b > kCoopThreshold) {  // the candidate of a long range, see flat_key_any
+      const uint32_t end = L.e;
+      L.anyhit = 0;
+      for (; L.b < end && L.best == kMiss; L.b = L.e) {
+        L.e = min(end, L.b + 32u);
+        lane_range<false, IND>(R, L, tests);
+      }
+      L.anyhit = 1;
+    } else {
+      lane_range<ANY, IND>(R, L, tests);
+    }
+  }
   lane_result(R, L, h);
 }
 
@@ -195,8 +210,9 @@ SHN_D int flat_test(float4 a, float4 b, float4 p0, float4 p1, float4 p2, float& 
 }
 
 // Ranges of more references than this are loaded once for all of the warp's
-// rays that wait on them; a ray that meets one of 2^24 is left to the general
-// walk.
+// rays that wait on them (kCoopThreshold where rays may be any-hit one by one:
+// their answer depends on it, see flat_key_any); a ray that meets one of 2^24
+// is left to the general walk.
 constexpr uint32_t kFlatLong = 63, kFlatHuge = 1u << 24;
 
 // The long ranges, listed from the end of W.own (lane and cell | length << 8,
@@ -215,22 +231,43 @@ SHN_D void flat_long(FlatWarpOf<K>& W, const Acc& acc, uint32_t count) {
       const uint32_t b = __shfl_sync(0xFFFFFFFFu, mine.y, j), len = __shfl_sync(0xFFFFFFFFu, mine.x, j) >> 8;
       const uint32_t scene = __shfl_sync(0xFFFFFFFFu, mscene, j);
       const Refs R = acc.refs(scene);
-      const uint32_t rays = todo & __ballot_sync(0xFFFFFFFFu, mine.y == b && (mine.x >> 8) == len && mscene == scene);
+      uint32_t rays = todo & __ballot_sync(0xFFFFFFFFu, mine.y == b && (mine.x >> 8) == len && mscene == scene);
       todo &= ~rays;
-      for (uint32_t i0 = 0; i0 < len; i0 += 32) {
+      for (uint32_t i0 = 0; i0 < len && rays; i0 += 32) {
         const bool in = i0 + lane < len;
         const uint32_t id = in ? __ldg(R.ridx + (b + i0 + lane)) : 0u;
         const float4* rec = R.rec + 3 * (size_t)id;
         const float4 p0 = __ldg(rec), p1 = __ldg(rec + 1), p2 = __ldg(rec + 2);
         for (uint32_t m = rays; m; m &= m - 1) {
-          const uint32_t slot = W.own[32 * K + 31 - (k0 + __ffs(m) - 1)].x & 255u, owner = slot & 31u;
-          if (ANY && *reinterpret_cast<volatile unsigned long long*>(&W.key[owner]) != ~0ull) continue;
+          const int r = __ffs(m) - 1;
+          const uint32_t slot = W.own[32 * K + 31 - (k0 + r)].x & 255u, owner = slot & 31u;
+          const bool first = MIXED && (__float_as_uint(W.d[owner].w) & 8u);
+          if (ANY || first) {
+            // answered by an earlier cell (or, ANY, by any cell)
+            const unsigned long long k = W.key[owner];
+            if (k != ~0ull && (ANY || (uint32_t)(k >> 61) < slot >> 5)) {
+              rays &= ~(1u << r);
+              continue;
+            }
+          }
           const float4 A = W.a[owner], B = W.b[owner];
           float t;
-          if (in && wt_test_p<3, 3, 3>(f4v(A), A.w, B.x, B.y, p0, p1, p2, kEps, B.w, t, __float_as_uint(B.z)))
-            atomicMin(&W.key[owner], MIXED && (__float_as_uint(W.d[owner].w) & 8u)
-                                         ? flat_key_any(t, slot >> 5, b + i0 + lane)
-                                         : flat_key(t, slot >> 5, id));
+          const bool hit =
+              in && wt_test_p<3, 3, 3>(f4v(A), A.w, B.x, B.y, p0, p1, p2, kEps, B.w, t, __float_as_uint(B.z));
+          if (ANY || first) {
+            const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
+            if (hits) {
+              // t is positive: its bits are in its order; references are in that of the ids
+              const uint32_t tb = hit ? __float_as_uint(t) : 0xFFFFFFFFu;
+              const uint32_t least = __ballot_sync(0xFFFFFFFFu, tb == __reduce_min_sync(0xFFFFFFFFu, tb));
+              if (lane == __ffs(least) - 1)
+                atomicMin(&W.key[owner], first ? flat_key_any(t, slot >> 5, b + i0 + lane) : flat_key(t, slot >> 5, id));
+              rays &= ~(1u << r);
+              __syncwarp();
+            }
+          } else if (hit) {
+            atomicMin(&W.key[owner], flat_key(t, slot >> 5, id));
+          }
         }
       }
     }
@@ -245,6 +282,8 @@ SHN_D void flat_long(FlatWarpOf<K>& W, const Acc& acc, uint32_t count) {
 template <bool ANY, bool MIXED = false, int K, class Acc, class Src, class Sink>
 SHN_D void flat_trace(FlatWarpOf<K>* smem, const Acc& acc, uint32_t n, bool uv, uint32_t* counter, Src&& src, Sink&& sink) {
   constexpr bool IND = true;
+  constexpr uint32_t kLong = MIXED ? kCoopThreshold : kFlatLong;
+  static_assert(kLong <= 63u, "the references of a window's short ranges have 14 bits");
   static_assert(Acc::kIndirect, "triangles are read by id");
   // rays reserved at a time, one reservation ahead of its use; fewer when there
   // are few rays for every warp
@@ -378,7 +417,7 @@ SHN_D void flat_trace(FlatWarpOf<K>* smem, const Acc& acc, uint32_t n, bool uv, 
           for (int q = 0; q < K; ++q) {
             if (r[q].y > r[q].x) {
               const uint32_t len = r[q].y - r[q].x;
-              packed += len > kFlatLong ? 1u << 23 : len << 9 | 1u;
+              packed += len > kLong ? 1u << 23 : len << 9 | 1u;
               again = again || len >= kFlatHuge;
             } else {
               skip = max(skip, (int)r[q].x - (K - q));
@@ -406,7 +445,7 @@ SHN_D void flat_trace(FlatWarpOf<K>* smem, const Acc& acc, uint32_t n, bool uv, 
           for (int q = 0; q < K; ++q) {
             if (r[q].y > r[q].x) {
               const uint32_t len = r[q].y - r[q].x;
-              if (len > kFlatLong) {
+              if (len > kLong) {
                 W.own[l--] = make_uint2((uint32_t)(32 * q + lane) | len << 8, r[q].x);
               } else {
                 W.own[k++] = make_uint2((uint32_t)(32 * q + lane) | f << 8, r[q].x - f);
@@ -421,7 +460,6 @@ SHN_D void flat_trace(FlatWarpOf<K>* smem, const Acc& acc, uint32_t n, bool uv, 
       }
       __syncwarp();
       // ---- test ------------------------------------------------------------------
-      if (nlong) flat_long<ANY, MIXED>(W, acc, nlong);
       // The triangle ids of kFlatGroups groups of 32 references are loaded together.
       uint32_t started = 0;
       for (uint32_t j0 = 0; j0 < sum; j0 += 32u * kFlatGroups) {
@@ -459,7 +497,8 @@ SHN_D void flat_trace(FlatWarpOf<K>* smem, const Acc& acc, uint32_t n, bool uv, 
           int hit = 0;
           float t;
           // (numbers go up with the cells and their references, so an any-hit
-          // ray's key from an earlier group stands)
+          // ray's key from an earlier group stands; the long ranges come later)
+          if (ANY || MIXED) __syncwarp();
           const bool done = (ANY || (MIXED && (bits & 8u))) && W.key[owner] != ~0ull;
           if (MIXED) __syncwarp();
           if (mine && !done)
@@ -477,6 +516,10 @@ SHN_D void flat_trace(FlatWarpOf<K>* smem, const Acc& acc, uint32_t n, bool uv, 
         }
       }
       __syncwarp();
+      if (nlong) {
+        flat_long<ANY, MIXED>(W, acc, nlong);
+        __syncwarp();
+      }
       // ---- the window's result ------------------------------------------------------
       // The cells are visited in order while the bound lies beyond the exit of
       // the one before, so a least t beyond the entry of its cell is the result

@@ -165,3 +165,102 @@ def test_mixed_requests(gpu, lambdas, rays):
                 assert np.all(np.abs(t[near] - t64[near]) <= 1e-4 * np.maximum(1.0, np.abs(t64[near])))
     finally:
         sv.close()
+
+
+@pytest.mark.parametrize("counts", [
+    (0, 3, 0, 100, 0, 40, 1, 0),       # short ranges before and behind long ones, a window's cells or two
+    (40, 0, 33, 1, 32, 31, 200, 64),
+    (1, 700, 1, 700, 1, 65, 0, 5),
+    (32, 33, 63, 64, 65, 95, 96, 97),  # around the lengths at which the engine changes
+])
+def test_any_hit_request_answer(gpu, counts):
+    """The triangle and t of an any-hit request are those of the first cell on the ray with a hit: there the
+    first reference that is hit of a range of up to 32, else the nearest hit of the first 32 references
+    that hold one.  Layers of triangles across the rays, sorted neither by depth nor by size."""
+    import torch
+
+    import shinobi_b200 as shn
+    r = np.random.RandomState(sum(counts))
+    layer = np.repeat(np.arange(8), counts)
+    r.shuffle(layer)
+    nt = layer.size + 8
+    x = np.empty(layer.size)
+    for c in range(8):  # inside the cell, 0.0004 apart or more
+        k = np.flatnonzero(layer == c)
+        x[k] = (c + 0.2 + 0.6 * (r.permutation(k.size) + 0.5) / max(1, k.size)) / 8.0
+    ang = np.sort(r.uniform(0, 2 * np.pi, (layer.size, 3)), axis=1)
+    tri = np.empty((nt, 3, 3))
+    tri[8:, :, 0] = x[:, None]
+    tri[8:, :, 1], tri[8:, :, 2] = 0.5 + 0.48 * np.cos(ang), 0.5 + 0.48 * np.sin(ang)
+    for k in range(8):  # the corners of the unit cube, so that the cells are its eighths
+        corner = np.array([k & 1, k >> 1 & 1, k >> 2 & 1], float)
+        tri[k] = corner + np.array([[0, 0, 0], [1e-3, 0, 0], [0, 1e-3, 0]]) * (1 - 2 * corner)
+    v = tri.reshape(-1, 3).astype(np.float32)
+    sc = type("S", (), {"vertices": v, "indices": np.arange(3 * nt, dtype=np.uint32).reshape(nt, 3),
+                        "num_triangles": nt})
+    lam = 8.5 ** 3 / nt
+    b = oracle.bounds(v, sc.indices)
+    res = oracle.resolution(nt, b, lam, 1, 1)
+    assert tuple(res) == (8, 8, 8) and np.allclose(b, [0, 0, 0, 1, 1, 1])
+    og = oracle.build_uniform(v, sc.indices, b, res)
+
+    n = 1500
+    cy, cz = r.randint(1, 7, n), r.randint(1, 7, n)
+    sign = np.where(r.rand(n) < 0.5, 1.0, -1.0)
+    org = np.empty((n, 3))
+    org[:, 0] = np.where(r.rand(n) < 0.7, np.where(sign > 0, -0.5, 1.5), r.uniform(0.0, 1.0, n))
+    org[:, 1], org[:, 2] = (cy + r.uniform(0.3, 0.7, n)) / 8.0, (cz + r.uniform(0.3, 0.7, n)) / 8.0
+    org = org.astype(np.float32)
+    d = np.stack([sign, r.uniform(-1e-3, 1e-3, n), r.uniform(-1e-3, 1e-3, n)], 1).astype(np.float32)
+    d[::5, 1:] = 0.0
+    tmax = np.where(r.rand(n) < 0.7, 8.0, r.uniform(0.2, 1.5, n)).astype(np.float32)
+
+    # every (ray, triangle) pair in float64; rays that pass an edge or a bound closely are left out
+    a = v.reshape(nt, 3, 3).astype(np.float64)[8:]
+    o64, d64 = org.astype(np.float64), d.astype(np.float64)
+    t = (a[None, :, 0, 0] - o64[:, None, 0]) / d64[:, None, 0]
+    p = o64[:, None, 1:] + t[..., None] * d64[:, None, 1:]
+    e = []
+    for k in range(3):
+        s, f = a[None, :, k, 1:], a[None, :, (k + 1) % 3, 1:]
+        e.append((f[..., 0] - s[..., 0]) * (p[..., 1] - s[..., 1]) - (f[..., 1] - s[..., 1]) * (p[..., 0] - s[..., 0]))
+    e = np.stack(e)
+    hit = (e > 0).all(0) & (t > 1e-5) & (t < tmax[:, None])
+    sure = ((np.abs(e) > 1e-5).all(0) & (np.abs(t - 1e-5) > 1e-4) & (np.abs(t - tmax[:, None]) > 1e-4)).all(1)
+    assert sure.sum() > n // 4
+
+    r8 = torch.zeros(n, 8).pin_memory()
+    r8[:, 0:3], r8[:, 3:6], r8[:, 6] = map(torch.from_numpy, (org, d, tmax))
+    got, gt = torch.zeros(n, dtype=torch.int32).pin_memory(), torch.zeros(n).pin_memory()
+    near, nt_ = torch.zeros(n, dtype=torch.int32).pin_memory(), torch.zeros(n).pin_memory()
+    sv = shn.Server(num_slots=1)
+    try:
+        sv.load_scene(0, sc, lam)
+        out = sv.run_schedule([sv.ray_request(shn._abi.SHN_REQ_ANY, 0, r8, got, gt),
+                               sv.ray_request(shn._abi.SHN_REQ_CLOSEST, 0, r8, near, nt_)], np.zeros(2))
+        assert not out.any()
+    finally:
+        sv.close()
+    got, gt = got.numpy().view(np.uint32), gt.numpy()
+    ref = oracle.trace_closest(og, org, d, tmax)
+    assert np.array_equal(near.numpy().view(np.uint32), ref[0])
+    assert np.array_equal(nt_.numpy().view(np.uint32), ref[1].view(np.uint32))
+    seen = set()
+    for i in np.flatnonzero(sure):
+        want = shn.SHN_MISS
+        for x_ in (range(8) if sign[i] > 0 else range(7, -1, -1)):
+            lo, hi = og.cells[x_ + 8 * cy[i] + 64 * cz[i]]
+            ids = og.indices[lo:hi].astype(np.int64) - 8
+            ids = ids[ids >= 0]
+            step = 1 if hi - lo <= 32 else 32
+            for k in range(0, ids.size, step):
+                part = ids[k:k + step][hit[i, ids[k:k + step]]]
+                if part.size:
+                    want = part[np.argmin(t[i, part])] + 8
+                    seen.add((step, k > 0))
+                    break
+            if want != shn.SHN_MISS:
+                assert abs(gt[i] - t[i, want - 8]) <= 1e-6 * 2.0
+                break
+        assert got[i] == want
+    assert len(seen) > 1

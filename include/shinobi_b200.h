@@ -651,6 +651,11 @@ shn_status shn_ctx_sync_status(shn_ctx* ctx, void* stream);
 #define SHN_FORCE_GRID_COMPACTION 2u
 #define SHN_FORCE_NOALLOC_SCAN 3u
 shn_status shn_debug_force_lookback_timeout(uint32_t target, shn_ctx* ctx, shn_grid* g);
+/* Failure-detection self test: the k-th device allocation of the context from
+ * now on (k = 1: the next one) fails as if there were no memory; 0 disarms.
+ * Returns the allocations that were left until the failure (0: it happened,
+ * or none was armed).  No counterpart in the reference. */
+uint32_t shn_debug_fail_alloc(shn_ctx* ctx, uint32_t k);
 /* Failure-detection self test: runs the look-back scan kernel with tile 0
  * never published, so tile 1's bounded wait must run out (about a second)
  * and report it.  Returns SHN_ERR_TIMEOUT when the wait ran out and the

@@ -183,6 +183,7 @@ SIGNATURES = {
     "shn_ctx_sync_status": ([vp, vp], i32),
     "shn_grid_sync_status": ([vp, vp], i32),
     "shn_batch_sync_status": ([vp, vp], i32),
+    "shn_debug_fail_alloc": ([vp, u32], u32),
     "shn_debug_force_lookback_timeout": ([u32, vp, vp], i32),
     "shn_dynamic_create": ([vp, vp, u32, vp, u32, u32, C.POINTER(GridParams), C.POINTER(vp)], i32),
     "shn_dynamic_render_frame": ([vp, vp, u32, vp, f32, C.POINTER(Camera), C.POINTER(DiParams), C.POINTER(Hits),

@@ -9,6 +9,10 @@
 namespace shn {
 
 cudaError_t dev_alloc(shn_ctx* ctx, void** p, size_t bytes, cudaStream_t st) {
+  uint32_t left = ctx->fail_alloc.load();
+  while (left && !ctx->fail_alloc.compare_exchange_weak(left, left - 1)) {
+  }
+  if (left == 1) return cudaErrorMemoryAllocation;
   if (ctx->budget) {
     const uint64_t now = ctx->used.fetch_add(bytes) + bytes;
     if (now > ctx->budget) {
@@ -595,6 +599,8 @@ shn_status shn_grid_sync_status(const shn_grid* g, void* stream) {
   if (g->ev1) cudaEventSynchronize(g->ev1);  // the build's tail, whatever its stream
   return read_and_clear(g->ctx, g->d_err, st, "grid");
 }
+
+uint32_t shn_debug_fail_alloc(shn_ctx* ctx, uint32_t k) { return ctx ? ctx->fail_alloc.exchange(k) : 0u; }
 
 shn_status shn_debug_force_lookback_timeout(uint32_t target, shn_ctx* ctx, shn_grid* g) {
   if (target == SHN_FORCE_CTX_SCAN) {

@@ -1104,16 +1104,28 @@ shn_status ensure_buf(shn_grid* g, DevBuf& b, size_t bytes, cudaStream_t st) {
   return ensure(g, &b.ptr, &b.bytes, bytes, st);
 }
 
+// Grows a buffer that a build can do without, if there is memory for it: a
+// failure leaves the buffer and the context's error text as they are.  Nothing
+// is allocated under a memory budget, where a build needs no more than what it
+// cannot do without.  The contents are not kept.
+void grow_optional(shn_grid* g, DevBuf& b, size_t bytes, cudaStream_t st) {
+  if (b.bytes >= bytes || g->ctx->budget) return;
+  void* p = nullptr;
+  const size_t want = bytes + bytes / 8;
+  if (dev_alloc(g->ctx, &p, want, st) != cudaSuccess) return;
+  dev_free(g->ctx, b.ptr, b.bytes, st);
+  b.ptr = p;
+  b.bytes = want;
+}
+
 // Room for the rows of n items in key buffer `buf`, which the sort does not
-// need before the emission has read them: what the buffer has and, in a
-// context without a memory budget, at least kRowsPerItem per item (the buffer
-// ends up about as large for the keys).  Under a budget nothing is allocated
-// for rows, so a build needs no more memory than its keys do.
+// need before the emission has read them: what the buffer has or can be given,
+// up to kRowsPerItem per item (8 GB at most; the buffer ends up about as large
+// for the keys).
 constexpr uint64_t kRowsPerItem = 6;
 
 uint64_t rows_room(shn_grid* g, int buf, uint64_t n, cudaStream_t st) {
-  const size_t want = std::min<uint64_t>(n * kRowsPerItem, 1ull << 30) * sizeof(uint2);
-  if (g->keys[buf].bytes < want && g->ctx->budget == 0 && ensure_buf(g, g->keys[buf], want, st) != SHN_OK) return 0;
+  grow_optional(g, g->keys[buf], std::min<uint64_t>(n * kRowsPerItem, 1ull << 30) * sizeof(uint2), st);
   return g->keys[buf].bytes / sizeof(uint2);
 }
 

@@ -36,6 +36,8 @@ struct shn_ctx {
   // failure-detection self test: the next context-level look-back scan
   // withholds its first tile (shn_debug_force_lookback_timeout)
   std::atomic<uint32_t> force_lookback{0};
+  // the allocations until the one that fails (shn_debug_fail_alloc), 0: none
+  std::atomic<uint32_t> fail_alloc{0};
   // One reference for the handle returned by shn_ctx_create and one per live
   // scene / grid / batch / server: the context (and its memory pool) is torn
   // down when the last of them is released, whatever the destruction order.

@@ -146,3 +146,43 @@ def test_build_over_budget_is_refused_and_context_survives(gpu):
     g = shn.Grid(ctx).build(soup, shn.grid_params(shn.SHN_GRID_UNIFORM))
     assert g.info().num_refs > 0
     ctx.close()
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+def test_every_allocation_of_a_build_may_fail(gpu, kind):
+    """Each device allocation of a first build fails in turn, as if there were no memory.  The build either
+    reports it, and the next one succeeds, or does without (room for kept rows): then its
+    result is the same and no error text stays behind."""
+    import shinobi_b200 as shn
+    sc = scenes.uniform_soup(5000, seed=4, offset_scale=0.03)
+    p = shn.grid_params(kind)
+    want = shn.Grid().build(shn.FaceSoup(sc.vertices, sc.indices), p).export()
+    refused = without = 0
+    for k in range(1, 64):
+        ctx = shn.Context(0)
+        soup = shn.FaceSoup(sc.vertices, sc.indices, ctx=ctx)
+        g = shn.Grid(ctx)
+        ctx.lib.shn_debug_fail_alloc(ctx.handle, k)
+        try:
+            g.build(soup, p)
+            failed = False
+        except shn.ShinobiError as e:
+            assert e.status == shn._abi.SHN_ERR_OOM
+            failed = True
+        if ctx.lib.shn_debug_fail_alloc(ctx.handle, 0):
+            assert not failed
+            break  # fewer than k allocations
+        if failed:
+            refused += 1
+            g.build(soup, p)
+        else:
+            without += 1
+            assert not ctx.lib.shn_ctx_last_error(ctx.handle)
+        got = g.export()
+        for name in ("cells", "leaves", "indices", "top_pairs"):
+            assert np.array_equal(got[name], want[name]), (k, name)
+        del g, soup
+        ctx.close()
+    else:
+        pytest.fail("a build of more than 63 allocations")
+    assert refused > 5 and without == 1 + kind

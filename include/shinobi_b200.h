@@ -456,6 +456,8 @@ shn_status shn_batch_autotune(shn_batch* b, const float* candidates, uint32_t nu
  *  sort_tile_keys[0 .. num_sort_tiles): keys per tile of the batch's
  *    onesweep passes (4096 or 6144), each timed as the batch's whole build
  *    (median of three) on the chosen grids; the fastest is kept.
+ *    0 entries: by the number of keys, 2048, 4096 or 6144 (2048 up to
+ *    606,208, 4096 up to twice that).
  * sah_cost (optional, num_scenes) receives the chosen candidate's SAH cost;
  * report (optional) the work done and the shape timings.  Synchronises. */
 typedef struct shn_autotune_config {
@@ -469,7 +471,7 @@ typedef struct shn_autotune_report {
   uint32_t timed_candidates;  /* (scene, lambda) builds timed */
   uint32_t blocks_per_sm;     /* chosen (0: occupancy limit) */
   float shape_ms[8];          /* median sample trace time per blocks_per_sm entry */
-  uint32_t sort_tile_keys;    /* chosen keys per onesweep tile */
+  uint32_t sort_tile_keys;    /* chosen keys per onesweep tile (0: by the number of keys) */
   float sort_tile_ms[4];      /* median whole-build time per sort_tile_keys entry */
 } shn_autotune_report;
 shn_status shn_batch_autotune_ex(shn_batch* b, const float* candidates, uint32_t num_candidates,

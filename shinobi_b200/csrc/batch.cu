@@ -57,7 +57,7 @@ struct shn_batch {
   float build_ms = 0.f;
   int blocks_closest = 0, blocks_any = 0;  // persistent grid sizes (computed before any capture)
   uint32_t bps_closest = 0;                // autotuned blocks per SM of the closest-hit trace (0: occupancy)
-  uint32_t sort_tile = 0;                  // autotuned keys per onesweep tile (0: 6144)
+  uint32_t sort_tile = 0;                  // autotuned keys per onesweep tile (0: by the number of keys)
 };
 
 namespace shn {
@@ -637,7 +637,7 @@ shn_status shn_batch_autotune_ex(shn_batch* b, const float* candidates, uint32_t
         rc = set_error(ctx, SHN_ERR_INVALID, "sort tile shapes: 4096 or 6144 keys (0: 6144)");
         break;
       }
-      b->sort_tile = tk == 6144 ? 0u : tk;
+      b->sort_tile = tk ? tk : 6144u;
       float t[3];
       for (int r = 0; r < 3 && rc == SHN_OK; ++r) {
         cudaEventRecord(e1, st);
@@ -670,7 +670,7 @@ shn_status shn_batch_autotune_ex(shn_batch* b, const float* candidates, uint32_t
     report->timed_candidates = timed;
     if (!nshapes) report->blocks_per_sm = b->bps_closest;
     memcpy(report->shape_ms, shape_ms, sizeof(shape_ms));
-    report->sort_tile_keys = b->sort_tile ? b->sort_tile : 6144u;
+    report->sort_tile_keys = b->sort_tile;
     memcpy(report->sort_tile_ms, tile_ms, sizeof(tile_ms));
   }
   return SHN_OK;

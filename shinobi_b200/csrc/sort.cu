@@ -389,8 +389,7 @@ uint64_t* onesweep_sort(uint64_t* buf0, uint64_t* buf1, uint32_t n, uint32_t lo_
     const uint32_t shift = lo_bit + plan.width * p;
     const uint32_t w = std::min(plan.width, plan.bits - plan.width * p);
     const uint32_t mask = (1u << w) - 1u;
-    // 4096-key tiles (8 per thread) are the autotuner's alternative tile shape
-    const int items = tile_keys == 4096u ? 8 : (tile_keys ? kPassItems : sort_items(n));
+    const int items = tile_keys ? (int)tile_keys / kSortBlock : sort_items(n);
     if (plan.width == 9) {
       if (items == 4) launch_pass<4, 2, 9>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);
       else if (items == 8) launch_pass<8, 2, 9>(src, dst, n, shift, mask, hist + p * kMaxBins, status, tickets + p, d_err, st);

@@ -141,3 +141,23 @@ def test_batch_build_with_4096_key_sort_tiles(gpu):
         ex = bt.export_scene(s, og.cells.shape[0], og.indices.size)
         assert np.array_equal(ex["cells"], og.cells)
         assert np.array_equal(ex["indices"], og.indices)
+
+
+@pytest.mark.parametrize("tris", [2000, 160_000, 300_000])  # 2048-, 4096- and 6144-key tiles by the number of keys
+def test_sort_tile_choice(gpu, tris):
+    """The report names the tile asked for (an entry of 0: 6144), and none (0) where the sorts go by the
+    number of keys; the grids are the same."""
+    import shinobi_b200 as shn
+    sc = scenes.uniform_soup(tris, seed=1)
+    bt = shn.Batch([sc])
+    cands = np.array([5.0], np.float32)
+    ref = None
+    for tiles, want in (((), 0), ((6144,), 6144), ((4096,), 4096), ((0,), 6144)):
+        rep = bt.autotune_ex(cands, expected_rays=[1000], sample_rays=1024, sort_tiles=tiles)[2]
+        bt.build()
+        n = bt.info()["num_pairs"]
+        assert {2000: n <= 606_208, 160_000: 606_208 < n <= 1_212_416, 300_000: n > 1_212_416}[tris]
+        assert rep["sort_tile_keys"] == want
+        ex = bt.export_scene(0, bt.info()["total_cells"], n)
+        ref = ref or ex
+        assert np.array_equal(ex["cells"], ref["cells"]) and np.array_equal(ex["indices"], ref["indices"])

@@ -8,12 +8,12 @@ namespace shn {
 
 namespace {
 
-template <bool ANY, int K>
+template <bool ANY, int K, bool COH>
 __global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : 6)
     k_flat_rays(const __grid_constant__ GridView G, RaysView R, uint32_t n, uint32_t* counter, uint32_t* otri,
                 float* ot, float* ou, float* ov, uint8_t* occ) {
   __shared__ FlatWarpOf<K> sm[kCoopBlock / 32];
-  flat_trace<ANY>(
+  flat_trace<ANY, false, false, COH>(
       sm, FlatGrid{&G}, n, ou || ov, counter,
       [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&, uint32_t&) {
         R.ray(i, o, d, tmax);
@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : 6)
     k_flat_camera(const __grid_constant__ GridView G, CamView cam, uint32_t image_id, uint32_t n, uint32_t* counter,
                   uint32_t* otri, float* ot, float* ou, float* ov) {
   __shared__ FlatWarpOf<K> sm[kCoopBlock / 32];
-  flat_trace<false>(
+  flat_trace<false, false, true>(
       sm, FlatGrid{&G}, n, ou || ov, counter,
       [&](uint32_t i, V3& o, V3& d, float& tmax, uint32_t&, uint32_t&) {
         o = cam.eye;
@@ -76,17 +76,18 @@ int flat_blocks(int num_sms, uint64_t n) {
 
 }  // namespace
 
-template <bool ANY, int K>
+template <bool ANY, int K, bool COH = false>
 static void flat_rays(const GridView& G, const RaysView& rays, uint32_t n, uint32_t* counter, const shn_hits& hits,
                       uint8_t* occ, int num_sms, cudaStream_t st) {
-  k_flat_rays<ANY, K><<<flat_blocks<k_flat_rays<ANY, K>>(num_sms, n), kCoopBlock, 0, st>>>(
+  k_flat_rays<ANY, K, COH><<<flat_blocks<k_flat_rays<ANY, K, COH>>(num_sms, n), kCoopBlock, 0, st>>>(
       G, rays, n, counter, hits.tri, hits.t, hits.u, hits.v, occ);
 }
 
 void launch_flat_closest(const GridView& G, const RaysView& rays, uint32_t n, uint32_t* counter, const shn_hits& hits,
                          int num_sms, cudaStream_t st) {
-  if (n < kFlatFew) flat_rays<false, kFlatAheadFew>(G, rays, n, counter, hits, nullptr, num_sms, st);
-  else flat_rays<false, kFlatAhead>(G, rays, n, counter, hits, nullptr, num_sms, st);
+  if (n <= kFlatAlone) flat_rays<false, kFlatAheadFew>(G, rays, n, counter, hits, nullptr, num_sms, st);
+  else if (n < kFlatFew) flat_rays<false, kFlatAheadFew, true>(G, rays, n, counter, hits, nullptr, num_sms, st);
+  else flat_rays<false, kFlatAhead, true>(G, rays, n, counter, hits, nullptr, num_sms, st);
 }
 
 void launch_flat_any(const GridView& G, const RaysView& rays, uint32_t n, uint32_t* counter, uint8_t* occ, int num_sms,

@@ -264,3 +264,52 @@ def test_any_hit_request_answer(gpu, counts):
                 break
         assert got[i] == want
     assert len(seen) > 1
+
+
+@pytest.mark.parametrize("what,tris,res,rays", [
+    ("ball", 30000, (21, 21, 21), 5003),     # empty cells around cells of thousands of references
+    ("ball", 30000, (90, 88, 91), 140001),   # up to ~200 references in a cell, short ranges around
+    ("large", 1500, (33, 32, 31), 20011),    # triangles of many cells, missing from some that they cross
+    ("large", 6000, (9, 10, 8), 4001),       # the same in long ranges
+    ("plates", 4000, (40, 3, 3), 3001),      # long thin triangles across whole rows of cells
+])
+def test_dense_cells(gpu, what, tris, res, rays):
+    """Closest and any hits, from arrays and from a camera, where cells are crowded or triangles are large
+    against them: bit for bit those of the oracle."""
+    import torch
+
+    import shinobi_b200 as shn
+    r = np.random.RandomState(tris + res[0])
+    if what == "ball":
+        c = r.normal(size=(tris, 1, 3))
+        c = 0.5 + 0.04 * c / np.linalg.norm(c, axis=2, keepdims=True) * r.uniform(0, 1, (tris, 1, 1)) ** (1 / 3)
+        c[::10] = r.uniform(0, 1, (len(c[::10]), 1, 3))
+        v = c + r.uniform(-0.004, 0.004, (tris, 3, 3))
+    elif what == "large":
+        v = r.uniform(0.2, 0.8, (tris, 1, 3)) + r.uniform(-0.2, 0.2, (tris, 3, 3))
+    else:
+        v = r.uniform(0.0, 1.0, (tris, 1, 3)) + r.uniform(-1, 1, (tris, 3, 3)) * np.array([0.5, 0.02, 0.02])
+    v = v.reshape(-1, 3).astype(np.float32)
+    idx = np.arange(3 * tris, dtype=np.uint32).reshape(-1, 3)
+    b = oracle.bounds(v, idx)
+    og = oracle.build_uniform(v, idx, b, np.array(res, np.int32))
+    g = shn.Grid().build(shn.FaceSoup(v, idx), shn.grid_params(shn.SHN_GRID_UNIFORM, res=res))
+    org, d, tmax = _rays(rays, b, seed=7)
+    near = np.arange(rays) % 3 != 0  # two of three rays aim at the crowd
+    aim = 0.5 + r.uniform(-0.05, 0.05, (rays, 3)) - org
+    aim /= np.maximum(1e-6, np.linalg.norm(aim, axis=1, keepdims=True))
+    d[near] = aim[near].astype(np.float32)
+    dev = [torch.from_numpy(x).cuda() for x in (org, d, tmax)]
+    h = g.trace_closest(*dev)
+    ref = oracle.trace_closest(og, org, d, tmax)
+    for name, x, y in zip(("tri", "t", "u", "v"), (h.tri, h.t, h.u, h.v), ref):
+        assert np.array_equal(x.cpu().numpy().view(np.uint32), np.ascontiguousarray(y).view(np.uint32)), name
+    assert (h.tri != -1).any()
+    occ = g.trace_any(*dev).cpu().numpy()
+    assert np.array_equal(occ, np.asarray(oracle.trace_any(og, org, d, tmax)[0]).astype(np.uint8))
+    cam = scenes.Camera((0.4, -0.7, 0.6), (0.1, 1.2, -0.1), (0.0, 0.0, 1.0), 30.0, 131, 89)
+    c = g.trace_primary(cam)
+    co, cd = oracle.primary_rays(cam)
+    ref = oracle.trace_closest(og, co, cd)
+    for name, x, y in zip(("tri", "t", "u", "v"), (c.tri, c.t, c.u, c.v), ref):
+        assert np.array_equal(x.cpu().numpy().view(np.uint32), np.ascontiguousarray(y).view(np.uint32)), name

@@ -335,12 +335,13 @@ class Grid:
 
     @staticmethod
     def _strided(org, dirs, tmax):
-        """Rays read in place: float32 device arrays (n, 3), (n, 3) and (n,) of any strides; None for others."""
+        """Rays read in place: float32 device arrays (n, 3), (n, 3) and (n,) of any strides; None for others (and
+        for views whose memory holds the negated values)."""
         torch = _torch()
         if (org.ndim != 2 or dirs.ndim != 2 or org.shape[1] < 3 or dirs.shape[1] < 3 or dirs.shape[0] < org.shape[0]
                 or (tmax is not None and (tmax.ndim != 1 or tmax.shape[0] < org.shape[0]))):
             return None
-        if any(x is not None and (x.dtype != torch.float32 or not x.is_cuda) for x in (org, dirs, tmax)):
+        if any(x is not None and (x.dtype != torch.float32 or not x.is_cuda or x.is_neg()) for x in (org, dirs, tmax)):
             return None
         o, d, so, sd = org.data_ptr(), dirs.data_ptr(), org.stride(), dirs.stride()
         r = _abi.Rays(*[o + 4 * k * so[1] for k in range(3)], *[d + 4 * k * sd[1] for k in range(3)],

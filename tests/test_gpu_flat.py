@@ -313,3 +313,23 @@ def test_dense_cells(gpu, what, tris, res, rays):
     ref = oracle.trace_closest(og, co, cd)
     for name, x, y in zip(("tri", "t", "u", "v"), (c.tri, c.t, c.u, c.v), ref):
         assert np.array_equal(x.cpu().numpy().view(np.uint32), np.ascontiguousarray(y).view(np.uint32)), name
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+def test_rays_in_negated_views(gpu, kind):
+    """Rays whose memory holds the negated values (the imaginary part of a conjugate) are not read in place."""
+    import torch
+
+    import shinobi_b200 as shn
+    sc = scenes.uniform_soup(5000, seed=3)
+    g = shn.Grid().build(shn.FaceSoup(sc.vertices, sc.indices), shn.grid_params(kind))
+    rays = [torch.from_numpy(x).cuda() for x in _rays(1003, oracle.bounds(sc.vertices, sc.indices), seed=5)]
+    neg = [torch.complex(torch.zeros_like(x), -x).conj().imag for x in rays]
+    assert all(x.is_neg() and torch.equal(x, y) for x, y in zip(neg, rays))
+    ref, occ = g.trace_closest(*rays), g.trace_any(*rays)
+    assert (ref.tri != -1).any()
+    for k in ((1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1)):
+        r = [neg[i] if k[i] else rays[i] for i in range(3)]
+        h = g.trace_closest(*r)
+        assert torch.equal(h.tri, ref.tri) and torch.equal(h.t.view(torch.int32), ref.t.view(torch.int32))
+        assert torch.equal(g.trace_any(*r), occ)

@@ -540,69 +540,69 @@ SHN_D uint64_t warp_range_cull_p(const Refs& G, V3 org, V3 cr, float Sx, float S
   uint32_t ntest = 0;
   bool done = false;
   for (uint32_t s0 = kb >> 5; s0 <= (ke >> 5) && !done; s0 += 32u) {
-  // the super-blocks the ray meets, one box per lane
-  const uint32_t sl = min(s0 + lane, ke >> 5);
-  const float4 smn = __ldg(G.sbox + 2 * (size_t)sl), smx = __ldg(G.sbox + 2 * (size_t)sl + 1);
-  uint32_t cand = __ballot_sync(0xFFFFFFFFu, s0 + lane <= (ke >> 5) && box_meets(org, cr, smn, smx, tbest));
-  const uint32_t sorder = ANY ? 0u : box_order(org, cr, smn, smx);
-  while (cand && !done) {
-    const uint32_t sbit = ANY ? (uint32_t)(__ffs(cand) - 1) : first_box(cand, sorder);
-    const uint32_t s = s0 + sbit;
-    cand &= ~(1u << sbit);
-    uint64_t wk = key;
+    // the super-blocks the ray meets, one box per lane
+    const uint32_t sl = min(s0 + lane, ke >> 5);
+    const float4 smn = __ldg(G.sbox + 2 * (size_t)sl), smx = __ldg(G.sbox + 2 * (size_t)sl + 1);
+    uint32_t cand = __ballot_sync(0xFFFFFFFFu, s0 + lane <= (ke >> 5) && box_meets(org, cr, smn, smx, tbest));
+    const uint32_t sorder = ANY ? 0u : box_order(org, cr, smn, smx);
+    while (cand && !done) {
+      const uint32_t sbit = ANY ? (uint32_t)(__ffs(cand) - 1) : first_box(cand, sorder);
+      const uint32_t s = s0 + sbit;
+      cand &= ~(1u << sbit);
+      uint64_t wk = key;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const uint64_t other = __shfl_xor_sync(0xFFFFFFFFu, wk, o);
-      wk = other < wk ? other : wk;
-    }
-    const float tw = wk == ~0ull ? tbest : __uint_as_float((uint32_t)(wk >> 32));
-    if (!ANY && tw < tbest && !box_meets(org, cr, __ldg(G.sbox + 2 * (size_t)s), __ldg(G.sbox + 2 * (size_t)s + 1), tw))
-      continue;
-    const uint32_t k = 32u * s + lane;
-    const bool need = k >= kb && k <= ke &&
-                      box_meets(org, cr, __ldg(G.cbox + 2 * (size_t)k), __ldg(G.cbox + 2 * (size_t)k + 1), tw);
-    uint32_t m = __ballot_sync(0xFFFFFFFFu, need);
-    while (m) {
-      const uint32_t k1 = 32u * s + (uint32_t)(__ffs(m) - 1);
-      m &= m - 1;
-      uint32_t k2 = ~0u;
-      if (!ANY && m) {
-        k2 = 32u * s + (uint32_t)(__ffs(m) - 1);
+      for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t other = __shfl_xor_sync(0xFFFFFFFFu, wk, o);
+        wk = other < wk ? other : wk;
+      }
+      const float tw = wk == ~0ull ? tbest : __uint_as_float((uint32_t)(wk >> 32));
+      if (!ANY && tw < tbest && !box_meets(org, cr, __ldg(G.sbox + 2 * (size_t)s), __ldg(G.sbox + 2 * (size_t)s + 1), tw))
+        continue;
+      const uint32_t k = 32u * s + lane;
+      const bool need = k >= kb && k <= ke &&
+                        box_meets(org, cr, __ldg(G.cbox + 2 * (size_t)k), __ldg(G.cbox + 2 * (size_t)k + 1), tw);
+      uint32_t m = __ballot_sync(0xFFFFFFFFu, need);
+      while (m) {
+        const uint32_t k1 = 32u * s + (uint32_t)(__ffs(m) - 1);
         m &= m - 1;
-      }
-      ntest += block_refs(k1, b, e) + (k2 != ~0u ? block_refs(k2, b, e) : 0u);
-      const uint32_t it = 32u * k1 + lane, it2 = 32u * k2 + lane;
-      const bool ok = it >= b && it < e;
-      const bool ok2 = !ANY && k2 != ~0u && it2 >= b && it2 < e;
-      bool hit = false;
-      float t;
-      if (ok) {
-        const float4 p0 = __ldg(G.rv0 + it), p1 = __ldg(G.rv1 + it), p2 = __ldg(G.rv2 + it);
-        if (wt_test_p<KX, KY, KZ>(org, Sx, Sy, Sz, p0, p1, p2, kEps, key == ~0ull ? tb : next_up(tb), t, perm)) {
-          const uint64_t c = ((uint64_t)__float_as_uint(t) << 32) | __float_as_uint(p0.w);
-          if (c < key) {
-            key = c;
-            tb = t;
-          }
-          hit = true;
+        uint32_t k2 = ~0u;
+        if (!ANY && m) {
+          k2 = 32u * s + (uint32_t)(__ffs(m) - 1);
+          m &= m - 1;
         }
-      }
-      if (ok2) {
-        const float4 p0 = __ldg(G.rv0 + it2), p1 = __ldg(G.rv1 + it2), p2 = __ldg(G.rv2 + it2);
-        if (wt_test_p<KX, KY, KZ>(org, Sx, Sy, Sz, p0, p1, p2, kEps, key == ~0ull ? tb : next_up(tb), t, perm)) {
-          const uint64_t c = ((uint64_t)__float_as_uint(t) << 32) | __float_as_uint(p0.w);
-          if (c < key) {
-            key = c;
-            tb = t;
+        ntest += block_refs(k1, b, e) + (k2 != ~0u ? block_refs(k2, b, e) : 0u);
+        const uint32_t it = 32u * k1 + lane, it2 = 32u * k2 + lane;
+        const bool ok = it >= b && it < e;
+        const bool ok2 = !ANY && k2 != ~0u && it2 >= b && it2 < e;
+        bool hit = false;
+        float t;
+        if (ok) {
+          const float4 p0 = __ldg(G.rv0 + it), p1 = __ldg(G.rv1 + it), p2 = __ldg(G.rv2 + it);
+          if (wt_test_p<KX, KY, KZ>(org, Sx, Sy, Sz, p0, p1, p2, kEps, key == ~0ull ? tb : next_up(tb), t, perm)) {
+            const uint64_t c = ((uint64_t)__float_as_uint(t) << 32) | __float_as_uint(p0.w);
+            if (c < key) {
+              key = c;
+              tb = t;
+            }
+            hit = true;
           }
         }
-      }
-      if (ANY && __any_sync(0xFFFFFFFFu, hit)) {
-        done = true;
-        break;
+        if (ok2) {
+          const float4 p0 = __ldg(G.rv0 + it2), p1 = __ldg(G.rv1 + it2), p2 = __ldg(G.rv2 + it2);
+          if (wt_test_p<KX, KY, KZ>(org, Sx, Sy, Sz, p0, p1, p2, kEps, key == ~0ull ? tb : next_up(tb), t, perm)) {
+            const uint64_t c = ((uint64_t)__float_as_uint(t) << 32) | __float_as_uint(p0.w);
+            if (c < key) {
+              key = c;
+              tb = t;
+            }
+          }
+        }
+        if (ANY && __any_sync(0xFFFFFFFFu, hit)) {
+          done = true;
+          break;
+        }
       }
     }
-  }
   }
   tests += ntest;
 #pragma unroll
@@ -745,103 +745,103 @@ SHN_D void group_cull_p(const Refs& G, const LaneG* park, unsigned long long* gk
   const float mytb0 = park[lane].tbest;
   uint32_t mycount = 0;
   for (uint32_t s0 = kb >> 5; s0 <= (ke >> 5) && live; s0 += 32u) {
-  // A few rays: the super-blocks any of them meets, one box per lane, ray by
-  // ray (one step per ray for 32 boxes); many rays: one step per box for all
-  // rays, below, costs less.
-  uint32_t cand = (ke >> 5) - s0 >= 31u ? 0xFFFFFFFFu : (2u << ((ke >> 5) - s0)) - 1u;
-  const uint32_t sl = min(s0 + lane, ke >> 5);
-  const float4 smn = __ldg(G.sbox + 2 * (size_t)sl), smx = __ldg(G.sbox + 2 * (size_t)sl + 1);
-  const V3 cr0 = cull_rcp(park[__ffs(gmask) - 1].rcp);
-  const uint32_t sorder = ANY ? 0u : box_order(o0, cr0, smn, smx);  // along the first ray
-  if (__popc(live) < __popc(cand)) {
-    bool met = false;
-    for (uint32_t m = live; m; m &= m - 1) {
-      const int r = __ffs(m) - 1;
-      const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + r);
-      const float tb = k == ~0ull ? park[r].tbest : __uint_as_float((uint32_t)(k >> 32));
-      met = met || box_meets(park[r].org, cull_rcp(park[r].rcp), smn, smx, tb);
-    }
-    cand &= __ballot_sync(0xFFFFFFFFu, met);
-  }
-  while (cand && live) {
-    const uint32_t sbit = ANY ? (uint32_t)(__ffs(cand) - 1) : first_box(cand, sorder);
-    const uint32_t s = s0 + sbit;
-    cand &= ~(1u << sbit);
-    bool in = false;
-    if (mine && ((live >> lane) & 1u)) {
-      const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + lane);
-      const float tb = k == ~0ull ? mytb0 : __uint_as_float((uint32_t)(k >> 32));
-      in = box_meets(myo, mycr, __ldg(G.sbox + 2 * (size_t)s), __ldg(G.sbox + 2 * (size_t)s + 1), tb);
-    }
-    const uint32_t rs = __ballot_sync(0xFFFFFFFFu, in);
-    if (!rs) continue;
-    const uint32_t kl = 32u * s + lane;
-    const bool kval = kl >= kb && kl <= ke;
-    float4 bmn = make_float4(0.f, 0.f, 0.f, 0.f), bmx = bmn;
-    if (kval) {
-      bmn = __ldg(G.cbox + 2 * (size_t)kl);
-      bmx = __ldg(G.cbox + 2 * (size_t)kl + 1);
-    }
-    uint32_t need = 0;  // rays that must test block kl
-    for (uint32_t m = rs; m; m &= m - 1) {
-      const int r = __ffs(m) - 1;
-      const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + r);
-      const float tb = k == ~0ull ? park[r].tbest : __uint_as_float((uint32_t)(k >> 32));
-      if (kval && box_meets(park[r].org, cull_rcp(park[r].rcp), bmn, bmx, tb)) need |= 1u << r;
-    }
-    uint32_t U = __ballot_sync(0xFFFFFFFFu, need != 0u);
-    const uint32_t border = ANY ? 0u : box_order(o0, cr0, bmn, bmx);
-    while (U && live) {
-      const int bl = ANY ? __ffs(U) - 1 : (int)first_box(U, border);
-      U &= ~(1u << bl);
-      uint32_t rays = __shfl_sync(0xFFFFFFFFu, need, bl) & live;
-      if (!rays) continue;
-      const uint32_t kk = 32u * s + (uint32_t)bl;
-      if (!ANY) {
-        // the bounds may have shrunk since: each lane looks at its own ray again
-        // (a step per block against a step per ray and block)
-        bool still = false;
-        if ((rays >> lane) & 1u) {
-          const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + lane);
-          still = k == ~0ull || box_meets(myo, mycr, __ldg(G.cbox + 2 * (size_t)kk), __ldg(G.cbox + 2 * (size_t)kk + 1),
-                                          __uint_as_float((uint32_t)(k >> 32)));
-        }
-        rays = __ballot_sync(0xFFFFFFFFu, still);
-        if (!rays) continue;
-      }
-      if ((rays >> lane) & 1u) mycount += block_refs(kk, b, e);
-      const uint32_t it = 32u * kk + lane;
-      const bool ok = it >= b && it < e;
-      float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0, p2 = p0;
-      if (ok) {
-        p0 = __ldg(G.rv0 + it);
-        p1 = __ldg(G.rv1 + it);
-        p2 = __ldg(G.rv2 + it);
-      }
-      V3 A, B, C;
-      if (SAME) {
-        A = sub(f4v(p0), o0);
-        B = sub(f4v(p1), o0);
-        C = sub(f4v(p2), o0);
-      }
-      for (uint32_t m = rays; m; m &= m - 1) {
+    // A few rays: the super-blocks any of them meets, one box per lane, ray by
+    // ray (one step per ray for 32 boxes); many rays: one step per box for all
+    // rays, below, costs less.
+    uint32_t cand = (ke >> 5) - s0 >= 31u ? 0xFFFFFFFFu : (2u << ((ke >> 5) - s0)) - 1u;
+    const uint32_t sl = min(s0 + lane, ke >> 5);
+    const float4 smn = __ldg(G.sbox + 2 * (size_t)sl), smx = __ldg(G.sbox + 2 * (size_t)sl + 1);
+    const V3 cr0 = cull_rcp(park[__ffs(gmask) - 1].rcp);
+    const uint32_t sorder = ANY ? 0u : box_order(o0, cr0, smn, smx);  // along the first ray
+    if (__popc(live) < __popc(cand)) {
+      bool met = false;
+      for (uint32_t m = live; m; m &= m - 1) {
         const int r = __ffs(m) - 1;
-        const float4 ra = *reinterpret_cast<const float4*>(&park[r].org);  // org, Sx
-        const float4 rb = *reinterpret_cast<const float4*>(&park[r].Sy);   // Sy, Sz, perm, tbest
         const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + r);
-        const float bound = k == ~0ull ? rb.w : __uint_as_float((uint32_t)(k >> 32) + 1u);
-        float t;
-        const bool hit =
-            ok && (SAME ? wt_test_t<KX, KY, KZ>(A, B, C, ra.w, rb.x, rb.y, kEps, bound, t, perm)
-                        : wt_test_p<KX, KY, KZ>(mk(ra.x, ra.y, ra.z), ra.w, rb.x, rb.y, p0, p1, p2, kEps, bound, t,
-                                                 KX == 3 ? __float_as_uint(rb.z) : perm));
-        if (hit) atomicMin(gkey + r, ((unsigned long long)__float_as_uint(t) << 32) | __float_as_uint(p0.w));
-        if (ANY) {
-          if (__any_sync(0xFFFFFFFFu, hit)) live &= ~(1u << r);
+        const float tb = k == ~0ull ? park[r].tbest : __uint_as_float((uint32_t)(k >> 32));
+        met = met || box_meets(park[r].org, cull_rcp(park[r].rcp), smn, smx, tb);
+      }
+      cand &= __ballot_sync(0xFFFFFFFFu, met);
+    }
+    while (cand && live) {
+      const uint32_t sbit = ANY ? (uint32_t)(__ffs(cand) - 1) : first_box(cand, sorder);
+      const uint32_t s = s0 + sbit;
+      cand &= ~(1u << sbit);
+      bool in = false;
+      if (mine && ((live >> lane) & 1u)) {
+        const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + lane);
+        const float tb = k == ~0ull ? mytb0 : __uint_as_float((uint32_t)(k >> 32));
+        in = box_meets(myo, mycr, __ldg(G.sbox + 2 * (size_t)s), __ldg(G.sbox + 2 * (size_t)s + 1), tb);
+      }
+      const uint32_t rs = __ballot_sync(0xFFFFFFFFu, in);
+      if (!rs) continue;
+      const uint32_t kl = 32u * s + lane;
+      const bool kval = kl >= kb && kl <= ke;
+      float4 bmn = make_float4(0.f, 0.f, 0.f, 0.f), bmx = bmn;
+      if (kval) {
+        bmn = __ldg(G.cbox + 2 * (size_t)kl);
+        bmx = __ldg(G.cbox + 2 * (size_t)kl + 1);
+      }
+      uint32_t need = 0;  // rays that must test block kl
+      for (uint32_t m = rs; m; m &= m - 1) {
+        const int r = __ffs(m) - 1;
+        const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + r);
+        const float tb = k == ~0ull ? park[r].tbest : __uint_as_float((uint32_t)(k >> 32));
+        if (kval && box_meets(park[r].org, cull_rcp(park[r].rcp), bmn, bmx, tb)) need |= 1u << r;
+      }
+      uint32_t U = __ballot_sync(0xFFFFFFFFu, need != 0u);
+      const uint32_t border = ANY ? 0u : box_order(o0, cr0, bmn, bmx);
+      while (U && live) {
+        const int bl = ANY ? __ffs(U) - 1 : (int)first_box(U, border);
+        U &= ~(1u << bl);
+        uint32_t rays = __shfl_sync(0xFFFFFFFFu, need, bl) & live;
+        if (!rays) continue;
+        const uint32_t kk = 32u * s + (uint32_t)bl;
+        if (!ANY) {
+          // the bounds may have shrunk since: each lane looks at its own ray again
+          // (a step per block against a step per ray and block)
+          bool still = false;
+          if ((rays >> lane) & 1u) {
+            const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + lane);
+            still = k == ~0ull || box_meets(myo, mycr, __ldg(G.cbox + 2 * (size_t)kk), __ldg(G.cbox + 2 * (size_t)kk + 1),
+                                            __uint_as_float((uint32_t)(k >> 32)));
+          }
+          rays = __ballot_sync(0xFFFFFFFFu, still);
+          if (!rays) continue;
+        }
+        if ((rays >> lane) & 1u) mycount += block_refs(kk, b, e);
+        const uint32_t it = 32u * kk + lane;
+        const bool ok = it >= b && it < e;
+        float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0, p2 = p0;
+        if (ok) {
+          p0 = __ldg(G.rv0 + it);
+          p1 = __ldg(G.rv1 + it);
+          p2 = __ldg(G.rv2 + it);
+        }
+        V3 A, B, C;
+        if (SAME) {
+          A = sub(f4v(p0), o0);
+          B = sub(f4v(p1), o0);
+          C = sub(f4v(p2), o0);
+        }
+        for (uint32_t m = rays; m; m &= m - 1) {
+          const int r = __ffs(m) - 1;
+          const float4 ra = *reinterpret_cast<const float4*>(&park[r].org);  // org, Sx
+          const float4 rb = *reinterpret_cast<const float4*>(&park[r].Sy);   // Sy, Sz, perm, tbest
+          const unsigned long long k = *reinterpret_cast<volatile const unsigned long long*>(gkey + r);
+          const float bound = k == ~0ull ? rb.w : __uint_as_float((uint32_t)(k >> 32) + 1u);
+          float t;
+          const bool hit =
+              ok && (SAME ? wt_test_t<KX, KY, KZ>(A, B, C, ra.w, rb.x, rb.y, kEps, bound, t, perm)
+                          : wt_test_p<KX, KY, KZ>(mk(ra.x, ra.y, ra.z), ra.w, rb.x, rb.y, p0, p1, p2, kEps, bound, t,
+                                                   KX == 3 ? __float_as_uint(rb.z) : perm));
+          if (hit) atomicMin(gkey + r, ((unsigned long long)__float_as_uint(t) << 32) | __float_as_uint(p0.w));
+          if (ANY) {
+            if (__any_sync(0xFFFFFFFFu, hit)) live &= ~(1u << r);
+          }
         }
       }
     }
-  }
   }
   if (mine) gend[lane] = b + mycount;
   __syncwarp();

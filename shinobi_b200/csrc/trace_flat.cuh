@@ -54,7 +54,9 @@ constexpr int kFlatGroups = 2;
 // wait for one ray's chain of windows and take longer ones: 200,000-triangle
 // soup, 1,021 / 16,000 / 64,000 / 130,000 rays 56 -> 50, 117 -> 86, 173 -> 159 and
 // 186 -> 170 us; from 200,000 rays on the shorter ones with a block more per SM
-// are as fast or faster (4.0M rays: 0.92 against 0.94 ms).
+// are as fast or faster (4.0M rays: 0.92 against 0.94 ms).  The single-grid
+// calls choose by this; bounces, batches and server launches, whose ray counts
+// vary, take kFlatAhead.
 constexpr int kFlatAhead = 6, kFlatAheadFew = 8;
 constexpr uint32_t kFlatFew = 1u << 17;
 

@@ -385,7 +385,10 @@ shn_status shn_shade_direct(const shn_grid* g, const shn_camera* cam, const shn_
 /* Work counters: when d_counters (2 x uint64, device) is non-NULL, later
  * trace calls on this grid run counting variants of their kernels and add
  * {cell visits, triangle tests} to it (for roofline accounting); NULL turns
- * counting off.  Not part of the reference interface. */
+ * counting off.  On uniform grids the counting variants walk cell by cell as
+ * the reference does: the hits are the same, the work counted is the
+ * reference's, not that of the kernels that run without counters.  Not part of
+ * the reference interface. */
 shn_status shn_grid_set_stats(shn_grid* g, uint64_t* d_counters);
 
 /* ---- dynamic scenes (DynamicRTEngine, src/Engine/DynamicRTEngine.h:49-158) -------

@@ -2,7 +2,7 @@
 the dense-cluster workload (1,048,576 triangles, leaf cells of tens of
 thousands of references), against the oracle, which tests every reference.
 
-The two-level build runs on the triangles in Morton order and the traversal
+The two-level build runs on the triangles in Hilbert order and the traversal
 skips 32-reference blocks whose box the ray's segment cannot meet.  Closest
 hits (triangle id and t) and any-hit flags must equal the oracle's bit for
 bit, for rays from a common eye (the grouped same-origin path), rays starting

@@ -9,7 +9,9 @@ namespace shn {
 namespace {
 
 template <bool ANY, int K, bool COH>
-__global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : 6)
+__global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks
+                                              : ANY || COH    ? kFlatBlocksFew
+                                                              : kFlatBlocksAlone)
     k_flat_rays(const __grid_constant__ GridView G, RaysView R, uint32_t n, uint32_t* counter, uint32_t* otri,
                 float* ot, float* ou, float* ov, uint8_t* occ) {
   __shared__ FlatWarpOf<K> sm[kCoopBlock / 32];
@@ -31,7 +33,7 @@ __global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : 6)
 }
 
 template <int K>
-__global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : 6)
+__global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : kFlatBlocksFew)
     k_flat_camera(const __grid_constant__ GridView G, CamView cam, uint32_t image_id, uint32_t n, uint32_t* counter,
                   uint32_t* otri, float* ot, float* ou, float* ov) {
   __shared__ FlatWarpOf<K> sm[kCoopBlock / 32];
@@ -52,7 +54,7 @@ __global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : 6)
 }
 
 template <class Rays, int K>
-__global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : 6)
+__global__ void __launch_bounds__(kCoopBlock, K == kFlatAhead ? kFlatBlocks : kFlatBlocksFew)
     k_flat_from_hits(const __grid_constant__ GridView G, const __grid_constant__ Rays R, const uint32_t* d_m,
                      uint32_t spp, uint32_t* counter) {
   __shared__ FlatWarpOf<K> sm[kCoopBlock / 32];

@@ -60,9 +60,12 @@ constexpr int kFlatGroups = 2;
 constexpr int kFlatAhead = 6, kFlatAheadFew = 8;
 constexpr uint32_t kFlatFew = 1u << 17;
 
-// Up to this many rays every one has a warp to itself, and there are no
-// neighbours to run side by side with (see COH).
+// Up to this many rays there are one or two to a warp: no neighbours to run side
+// by side with (see COH), and fewer blocks per SM, whose registers keep the chain
+// of windows free of spills (300 to 4,000 rays on a 65,536-triangle soup 2 us of
+// 40 to 48 less than at 6 blocks; 3 blocks the same, 5 a microsecond more).
 constexpr uint32_t kFlatAlone = 1u << 12;
+constexpr int kFlatBlocksAlone = 4, kFlatBlocksFew = 6;
 
 // Shared memory of one warp.  The rays live here, not in registers: the walk
 // loads and stores what it needs, so that the tests have the registers.  Every
